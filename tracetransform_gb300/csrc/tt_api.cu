@@ -73,6 +73,8 @@ struct FftTables {
     int M = 0;
     float2 *chirp = nullptr, *filt = nullptr, *twid = nullptr;
     float *lin = nullptr;
+    // the column-pair transforms' (where tt::fft_pair_fits(M))
+    float2 *filt_rev = nullptr, *tw = nullptr;
 };
 
 // A gather-capable CUDA array holding a source image (texel (u, v) = image
@@ -450,8 +452,27 @@ struct tt_plan {
         TT_CHECK(upload(&t.filt, filt));
         TT_CHECK(upload(&t.twid, twid));
         TT_CHECK(upload(&t.lin, lin));
+        if (tt::fft_pair_fits(M)) {
+            std::vector<float2> rev(M), tw(std::max<size_t>(tt::fft_twiddles(M), 1));
+            tt::fft_tables(M, filt.data(), rev.data(), tw.data());
+            TT_CHECK(upload(&t.filt_rev, rev));
+            TT_CHECK(upload(&t.tw, tw));
+        }
         fft[n] = t;
         *out = &fft[n];
+        return TT_OK;
+    }
+
+    // The tables of a column pair's chirp-z transform; *M its length.
+    tt_status get_chirp(int n, tt::ChirpTables *out, int *M) {
+        const FftTables *f;
+        TT_CHECK(get_fft(n, &f));
+        const float2 *tw;
+        TT_CHECK(get_p3dft(n, &tw, &out->ck));
+        out->chirp = f->chirp;
+        out->filt = f->filt_rev;
+        out->tw = f->tw;
+        *M = f->M;
         return TT_OK;
     }
 
@@ -630,32 +651,17 @@ tt_status run_circus_stacks(tt_plan *p, const float *d_sino, int rows, int cols,
                             const tt_pfunctional *pf, int n_p, unsigned need, float *d_out,
                             cudaStream_t st) {
     if ((need & (1u << 3)) && rows > tt::kP3DftMaxRows) {
-        // P3 of long columns: the chirp-z FFT kernel (its accumulation error
-        // does not grow with the column as the direct DFT's does), the rest here
-        CircusArgs a{};
-        a.sino = d_sino;
-        a.rows = rows;
-        a.cols = cols;
-        a.n_sino = n_sino;
-        a.n_p = n_p;
-        for (int i = 0; i < n_p; i++)
-            a.kind[i] = pf[i].kind;
-        a.need = 1u << 3;
-        a.out = d_out;
-        int sl = 1;
-        while (sl < rows)
-            sl <<= 1;
-        a.sort_len = sl;
-        const FftTables *f;
-        TT_CHECK(p->get_fft(rows, &f));
-        a.M = f->M;
-        a.chirp = f->chirp;
-        a.filt = f->filt;
-        a.twid = f->twid;
-        a.lin = f->lin;
-        if (tt::circus_smem_bytes(a) > 227 * 1024)
+        // P3 of long columns: chirp-z transforms of column pairs (whose
+        // accumulation error does not grow with the column as the direct
+        // DFT's does), the rest here
+        tt::ChirpTables t{};
+        int M = 0, kind[tt::kMaxP];
+        if (tt::p3_fft_length(rows) > 16384) // its buffer exceeds shared memory
             return fail(TT_ERR_UNSUPPORTED, "sinogram length %d exceeds the FFT buffers", rows);
-        TT_CUDA(tt::launch_circus(a, st));
+        TT_CHECK(p->get_chirp(rows, &t, &M));
+        for (int i = 0; i < n_p; i++)
+            kind[i] = pf[i].kind;
+        TT_CUDA(tt::launch_p3_fft(d_sino, rows, cols, n_sino, kind, n_p, t, M, d_out, st));
         need &= ~(1u << 3);
         if (!(need & ((1u << 1) | (1u << 2))))
             return TT_OK;
@@ -1204,18 +1210,21 @@ static tt_status circus_backward_impl(tt_plan *plan, const T *d_sino, int rows, 
     const int *kinds;
     TT_CHECK(p->get_kinds(pf, n_p, &kinds));
     if (sizeof(T) == sizeof(float)) {
-        const FftTables *f;
-        TT_CHECK(p->get_fft(rows, &f)); // the forward's float linspace and FFT tables
-        lin = (const T *)f->lin;
-        // both DFTs of a column by the chirp-z FFT where its M-point buffer
+        // both DFTs of a column pair by the chirp-z transform where its buffer
         // fits in shared memory, else the direct sums below
-        if (tt::circus_backward_fft_fits(rows, f->M)) {
+        if (tt::fft_pair_fits(tt::p3_fft_length(rows))) {
+            tt::ChirpTables t{};
+            int M = 0;
+            TT_CHECK(p->get_chirp(rows, &t, &M));
             TT_CUDA(tt::launch_circus_backward_fft(
                 (const float *)d_sino, rows, cols, n_sino, kinds, n_p,
-                (const float *)d_grad_circus, f->chirp, f->filt, f->twid, f->M, f->lin,
-                (float *)d_grad_sino, pick_stream(p, stream)));
+                (const float *)d_grad_circus, t, M, (float *)d_grad_sino,
+                pick_stream(p, stream)));
             return TT_OK;
         }
+        const FftTables *f;
+        TT_CHECK(p->get_fft(rows, &f)); // the forward's float linspace
+        lin = (const T *)f->lin;
         TT_CHECK(p->get_dft<T>(rows, &cosv, &sinv));
     } else {
         const double *l;

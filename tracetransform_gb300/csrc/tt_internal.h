@@ -47,6 +47,17 @@ inline bool interior_source(int n, int row_off, int col_off, int rows, int cols)
     return row_off >= 2 && col_off >= 2 && row_off + rows <= n - 1 && col_off + cols <= n - 1;
 }
 
+// The tables of a chirp-z column pair (tt_fft.cuh; device pointers, one set per
+// column length n and transform length M).
+struct ChirpTables {
+    const float2 *chirp; // n: exp(-i pi j^2 / n)
+    const float2 *filt;  // M: the convolution filter in digit-reversed order
+    const float2 *tw;    // the passes' twiddles
+    const float *ck;     // n / 2 + 1: trapz weights of the P3 bins
+};
+// Transform lengths the column-pair kernels take (shorter ones: direct sums).
+inline bool fft_pair_fits(int M) { return M >= 64 && M <= 16384; }
+
 // P-functionals over stacked sinograms.
 struct CircusArgs {
     const float *sino; // n_sino x cols x rows
@@ -103,6 +114,10 @@ size_t p3_tc_table_floats(int n);
 cudaError_t launch_p3_tc_tables(int n, const float2 *tw, float *out, cudaStream_t st);
 // Longest column whose P3 the direct DFT computes (longer ones: the FFT kernel).
 constexpr int kP3DftMaxRows = 2048;
+// P3 of longer columns by the chirp-z transform of column pairs, into entries
+// p with kind[p] == 3 of out (n_sino x n_p x cols); only where fft_pair_fits(M).
+cudaError_t launch_p3_fft(const float *sino, int rows, int cols, int n_sino, const int *kind,
+                          int n_p, const ChirpTables &t, int M, float *out, cudaStream_t st);
 // P3 frequency tiles of a column length n.
 int p3_freq_tiles(int n);
 size_t circus_warp_smem_bytes(int n_max);
@@ -115,6 +130,16 @@ cudaError_t launch_circus_stacks(const CircusStackArgs &a, size_t smem, cudaStre
 int p3_fft_length(int n);
 void p3_tables(int n, float2 *chirp, float2 *filt, float2 *twid, float *lin,
                std::complex<double> *work);
+// Tables of the radix-16 transform (tt_fft.cuh) of length m = 2^e >= 64: the
+// filter in digit-reversed order (m) and the passes' twiddles.
+inline int fft_lead_radix(int m) {
+    int e = 0;
+    while ((1 << e) < m)
+        e++;
+    return 1 << (((e - 1) & 3) + 1);
+}
+size_t fft_twiddles(int m);
+void fft_tables(int m, const float2 *filt, float2 *filt_rev, float2 *tw);
 
 // Rotation (cos(-theta), sin(-theta)) of an angle in degrees and the T3-T5
 // kernels (3 n entries) as the reference rounds them (tt_tables.cu).
@@ -153,16 +178,11 @@ cudaError_t launch_circus_backward(const T *sino, int rows, int cols, int n_sino
                                    const int *d_kinds, int n_p, const T *grad_circus,
                                    const T *cosv, const T *sinv, const T *lin, T *out,
                                    cudaStream_t st);
-// The float P-stage adjoint by the chirp-z identity on the forward's FFT
-// tables (chirp, filter, twiddles of length M); cudaErrorInvalidValue when
-// its shared memory (circus_backward_fft_smem) exceeds the device's.
+// The float P-stage adjoint by the chirp-z identity (transform length M,
+// tables t); only where fft_pair_fits(M).
 cudaError_t launch_circus_backward_fft(const float *sino, int rows, int cols, int n_sino,
                                        const int *d_kinds, int n_p, const float *grad_circus,
-                                       const float2 *chirp, const float2 *filt,
-                                       const float2 *twid, int M, const float *lin, float *out,
-                                       cudaStream_t st);
-size_t circus_backward_fft_smem(int rows, int M);
-bool circus_backward_fft_fits(int rows, int M);
+                                       const ChirpTables &t, int M, float *out, cudaStream_t st);
 template <typename T>
 cudaError_t launch_sino_backward(const T *grad_sino, const int *medians, int n_images, int n,
                                  int n_angles, unsigned long long tf_code, int n_t, T *params,

@@ -71,6 +71,39 @@ void p3_tables(int n, float2 *chirp, float2 *filt, float2 *twid, float *lin,
         lin[p] = (float)(-1 + p * 2.0 / (n - 1));
 }
 
+// The position-to-frequency map of the radix-16 passes (tt_fft.cuh) and
+// their twiddles: filt_rev[k * (m / 16) + b] = filt[frequency at position
+// 16 b + k]; tw holds, per pass of sub-length l and radix r (the leading one
+// 2, 4, 8 or 16, then 16s; none for l = 16), exp(-2 pi i j k / l) at
+// (k - 1) (l / r) + j.
+size_t fft_twiddles(int m) {
+    size_t total = 0;
+    for (int l = m, r = fft_lead_radix(m); l > 16; l /= r, r = 16)
+        total += (size_t)(r - 1) * (l / r);
+    return total;
+}
+
+void fft_tables(int m, const float2 *filt, float2 *filt_rev, float2 *tw) {
+    const int r1 = fft_lead_radix(m);
+    for (int p = 0; p < m; p++) {
+        int f = 0, weight = 1, rest = p;
+        for (int l = m, r = r1; l > 1; l /= r, r = 16) {
+            f += weight * (rest / (l / r)); // this pass's output digit
+            rest %= l / r;
+            weight *= r;
+        }
+        filt_rev[(size_t)(p % 16) * (m / 16) + p / 16] = filt[f];
+    }
+    for (int l = m, r = r1; l > 16; l /= r, r = 16) {
+        const int s = l / r;
+        for (int k = 1; k < r; k++)
+            for (int j = 0; j < s; j++) {
+                const double a = -2.0 * M_PI * ((double)j * k) / l;
+                *tw++ = make_float2((float)std::cos(a), (float)std::sin(a));
+            }
+    }
+}
+
 // pad() of c++/src/auxiliary.cpp:257-275: side N of the zero frame that holds
 // every rotation of a rows x cols image, and the image's offset inside it
 // (the reference's float origin and hypot arithmetic).
