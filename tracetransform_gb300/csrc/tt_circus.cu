@@ -18,8 +18,9 @@
 // P-functionals: P1, P2 by bitonic sort, P3 by the chirp-z (Bluestein)
 // identity on a power-of-two shared-memory FFT, and the Hermite projections
 // on a host-built basis psi_order(z(p)).
-// zscore_kernel follows c++/src/auxiliary.cpp:277-318 in the reference's own
-// order: a float mean, a double sum of squared float differences, n - 1.
+// zscore_kernel gives the value of c++/src/auxiliary.cpp:277-318 in the
+// reference's own order: a float mean, a double sum of squared float
+// differences, n - 1.
 #include <climits>
 
 #include "tt_common.cuh"
@@ -32,26 +33,90 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// z-score of one vector by one block, in the reference's order.
-__device__ __forceinline__ void zscore_vector(const float *__restrict__ x, int len,
-                                              float *__restrict__ z) {
-    __shared__ float s_mean, s_std;
-    if (threadIdx.x == 0) {
-        float sum = 0.f;
-        for (int i = 0; i < len; i++)
-            sum = __fadd_rn(sum, x[i]);
-        const float mean = __fdiv_rn(sum, (float)len);
-        double acc = 0.0;
-        for (int i = 0; i < len; i++) {
-            const double d = (double)__fsub_rn(x[i], mean);
-            acc = __dadd_rn(acc, __dmul_rn(d, d));
+// z-score of one vector by one warp: the value the reference's order gives
+// (a float sum for the mean, a double sum of squares), bit for bit.  The
+// float sum has to run in that order (its rounding is the result): the warp
+// stages 512 elements at a time (16 loads in flight per lane; waiting for each
+// 32 in turn cost more than the additions) and every lane adds them in turn.  The double sum is needed only up to the rounding of
+// the float standard deviation: any order of len non-negative terms ends
+// within (len - 1) 2^-53 of the exact sum, so the strided sum brackets the
+// ordered one.  Of the floats around a float estimate of sqrt(sum / (len -
+// 1)), one lane each, the result is the one whose rounding interval --
+// (midpoint to the float below, midpoint to the float above), exact in
+// double, as are their squares -- holds the bracket widened to 2 len + 64
+// units, which covers the roundings of the reference's division and square
+// root too.  When none does (a few vectors in a million, or NaN) the ordered
+// sum is formed.  Double-precision division and square root, whose many
+// dependent steps on the narrow FP64 pipe cost more than the sums, run there
+// only.  18 vectors of 360: 7.3 us (44 us with one thread doing all of it; 90:
+// 3.8 from 15.6 us, 720: 10.1 from 85 us).
+__device__ __forceinline__ void zscore_vector(const float *x, int len, float *z) {
+    __shared__ __align__(16) float s_x[512];
+    const int lane = threadIdx.x & 31;
+    float sum = 0.f;
+    for (int b = 0; b < len; b += 512) {
+        const int cnt = min(len - b, 512);
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            v[u] = lane + 32 * u < cnt ? x[b + lane + 32 * u] : 0.f;
+        __syncwarp(); // the previous 512 are read
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            s_x[lane + 32 * u] = v[u];
+        __syncwarp();
+        int i = 0;
+#pragma unroll 4
+        for (; i + 8 <= cnt; i += 8) {
+            const float4 t = *reinterpret_cast<const float4 *>(s_x + i);
+            const float4 w = *reinterpret_cast<const float4 *>(s_x + i + 4);
+            sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, t.x), t.y), t.z), t.w);
+            sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, w.x), w.y), w.z), w.w);
         }
-        s_mean = mean;
-        s_std = (float)sqrt(acc / (double)(len - 1));
+        for (; i < cnt; i++)
+            sum = __fadd_rn(sum, s_x[i]);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < len; i += blockDim.x)
-        z[i] = __fdiv_rn(__fsub_rn(x[i], s_mean), s_std);
+    const float mean = __fdiv_rn(sum, (float)len);
+    double acc = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < len; i += 32) {
+        const double d = (double)__fsub_rn(x[i], mean);
+        acc = fma(d, d, acc); // d d is exact in double: one rounding, as an add
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        acc += __shfl_xor_sync(TT_FULL_MASK, acc, o);
+    float sd = 0.f;
+    if (acc != 0.0) { // (0: every difference is 0, in any order)
+        // lane l tests the float l - 2 steps from the estimate (formed from
+        // acc 4^-q, in [1, 4), as acc itself may exceed the floats)
+        const int hi = __double2hiint(acc), q = (((hi >> 20) & 0x7ff) - 1023) >> 1;
+        const float part = (float)__hiloint2double(hi - 2 * q * (1 << 20), __double2loint(acc));
+        const float est = q < -100 || q > 100
+                              ? 0.f
+                              : sqrtf(__fdividef(part, (float)(len - 1))) *
+                                    __int_as_float((127 + q) << 23);
+        sd = __int_as_float(__float_as_int(est) + lane - 2);
+        const double mid = 0.5 * ((double)sd + (double)__int_as_float(__float_as_int(sd) + 1));
+        const double low = 0.5 * ((double)sd + (double)__int_as_float(__float_as_int(sd) - 1));
+        const double e = (2.0 * len + 64.0) * 1.1102230246251565e-16, k = (double)(len - 1);
+        const bool hit = est > 1e-30f && est < 1e30f && low * low * k < acc * (1.0 - e) &&
+                         acc * (1.0 + e) < mid * mid * k;
+        const unsigned ball = __ballot_sync(TT_FULL_MASK, hit);
+        sd = __shfl_sync(TT_FULL_MASK, sd, ball ? __ffs(ball) - 1 : 0);
+        if (!ball) {
+            acc = 0.0;
+            for (int i = 0; i < len; i++) {
+                const double d = (double)__fsub_rn(x[i], mean);
+                acc = __dadd_rn(acc, __dmul_rn(d, d));
+            }
+            sd = (float)sqrt(acc / (double)(len - 1));
+        }
+    } else if (len == 1) {
+        sd = __int_as_float(0x7fc00000); // 0 / 0
+    }
+    for (int i = lane; i < len; i += 32)
+        z[i] = __fdiv_rn(__fsub_rn(x[i], mean), sd);
 }
 
 // All requested P-functionals of column colidx of sinogram sidx.  Every thread
@@ -226,14 +291,15 @@ __global__ void __launch_bounds__(kThreads) circus_kernel(const CircusArgs a) {
 }
 
 // z-score of vectors of varying length: vector v is in[off[v] .. off[v] + len[v]).
-__global__ void zscore_batch_kernel(const float *__restrict__ in, const long long *__restrict__ off,
-                                    const int *__restrict__ len, float *__restrict__ out) {
+// One warp per CTA: few vectors then spread over the SMs.
+__global__ void __launch_bounds__(32)
+zscore_batch_kernel(const float *in, const long long *__restrict__ off,
+                    const int *__restrict__ len, float *out) {
     const long long o = off[blockIdx.x];
     zscore_vector(in + o, len[blockIdx.x], out + o);
 }
 
-__global__ void zscore_kernel(const float *__restrict__ in, int len,
-                              float *__restrict__ out) {
+__global__ void __launch_bounds__(32) zscore_kernel(const float *in, int len, float *out) {
     zscore_vector(in + (size_t)blockIdx.x * len, len, out + (size_t)blockIdx.x * len);
 }
 
@@ -971,7 +1037,7 @@ cudaError_t launch_zscore(const float *in, int n_vec, int len, float *out,
                           cudaStream_t stream) {
     if (n_vec <= 0 || len <= 0)
         return cudaSuccess;
-    zscore_kernel<<<n_vec, 128, 0, stream>>>(in, len, out);
+    zscore_kernel<<<n_vec, 32, 0, stream>>>(in, len, out);
     return cudaGetLastError();
 }
 
@@ -979,7 +1045,7 @@ cudaError_t launch_zscore_batch(const float *in, const long long *off, const int
                                 int n_vec, float *out, cudaStream_t stream) {
     if (n_vec <= 0)
         return cudaSuccess;
-    zscore_batch_kernel<<<n_vec, 128, 0, stream>>>(in, off, len, out);
+    zscore_batch_kernel<<<n_vec, 32, 0, stream>>>(in, off, len, out);
     return cudaGetLastError();
 }
 
