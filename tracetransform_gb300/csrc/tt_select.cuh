@@ -1,4 +1,4 @@
-// tt_select.cuh -- weighted selection used by T6 and T7.
+// tt_select.cuh -- weighted selection used by T6, T7 and P2.
 //
 // TFunctional6/7 (c++/src/functionals.cpp:226-276) sort a key sequence,
 // accumulate sqrt-weights in sorted order and return the key at the first
@@ -6,18 +6,25 @@
 // the smallest key k with 2 * W(<= k) >= W, so no sort is needed:
 //
 //   1. weights become u32 fixed point (2^-30 of a power-of-two bound on the
-//      total), summed exactly and deterministically by integer atomics;
+//      total, so twice any sum fits 32 bits), summed exactly and
+//      deterministically by integer atomics;
 //   2. a 256-bin histogram linear in the key over [klo, khi] locates the bin
 //      holding the crossing (bins are monotone in the key);
-//   3. the keys of that bin are compacted into a 64-entry list, sorted by a
-//      warp bitonic network and scanned exactly; if the bin holds more than
-//      64 keys the interval shrinks to that bin's key range and step 2
-//      repeats (a bin whose keys are all equal is the answer).
+//   3. the entries of that bin are collected, and each lane adds up the
+//      weights of the entries up to its own: the smallest that qualifies is
+//      the answer.  A bin of more than kSelList entries is refined first:
+//      its key range takes the histogram's place and step 2 repeats (a bin
+//      whose keys are all equal is the answer).
 //
-// One warp per line.  Elements are the line's stored rows [b, e) at
-// x[row - jlo]; every other row is a zero sample (key 0, weight 0), which
-// cannot move the crossing unless all weights are zero, in which case the
-// reference returns its smallest key, 0.
+// One warp per line.  What bounds it is the instruction count: a histogram
+// pass and a collecting pass over half the line, each with as little per
+// element as it needs -- bins by one multiply-add into the mantissa of 2^23,
+// weights (a square root each) only in the histogram pass and for the few
+// collected entries -- and the fixed work per line.  The collected list takes
+// the histogram's place in shared memory.  1024^2 x 360 angles, T0-T7: 2.55 ms,
+// of which T6 and T7 1.17 (3.21 and 1.79 with the bins recomputed by
+// conversions and the weights in both passes, 64-bit scans and a 64-entry
+// bitonic sort).
 #pragma once
 
 #include "tt_common.cuh"
@@ -25,187 +32,14 @@
 namespace tt {
 
 constexpr int kSelBins = 256;
-constexpr int kSelList = 64;
+constexpr int kSelList = 192; // collected entries (in the histogram's place)
 
-struct SelScratch {
-    unsigned hist[kSelBins];
-    unsigned key[kSelList];
-    unsigned w[kSelList];
+struct __align__(16) SelScratch {
+    union {
+        unsigned hist[kSelBins];
+        uint2 list[kSelList]; // key bits, then the sample's bits or its weight
+    };
 };
-
-// Smallest bin d with 2 * (below + sum_{d' <= d} h[d']) >= total; adds the
-// weight of the bins before d to *below.
-__device__ __forceinline__ int sel_pick_bin(const unsigned *h, unsigned long long *below,
-                                            unsigned long long total, int lane) {
-    constexpr int per = kSelBins / 32;
-    unsigned run = 0;
-#pragma unroll
-    for (int k = 0; k < per; k++)
-        run += h[lane * per + k];
-    unsigned long long inc = run;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long t = __shfl_up_sync(TT_FULL_MASK, inc, d);
-        if (lane >= d)
-            inc += t;
-    }
-    unsigned long long cum = *below + inc - run;
-    int kfirst = per;
-    unsigned long long before = cum, last_before = cum;
-#pragma unroll
-    for (int k = 0; k < per; k++) {
-        const unsigned hk = h[lane * per + k];
-        if (k == per - 1)
-            last_before = cum;
-        if (kfirst == per && 2ull * (cum + hk) >= total) {
-            kfirst = k;
-            before = cum;
-        }
-        cum += hk;
-    }
-    const unsigned ball = __ballot_sync(TT_FULL_MASK, kfirst < per);
-    const int ln = ball ? __ffs(ball) - 1 : 31;
-    const int kk = __shfl_sync(TT_FULL_MASK, ball ? kfirst : per - 1, ln);
-    *below = __shfl_sync(TT_FULL_MASK, ball ? before : last_before, ln);
-    return ln * per + kk;
-}
-
-// Bitonic sort of 64 (key, weight) pairs held two per lane (element i in
-// lane i % 32, register i / 32), ascending by key.
-__device__ __forceinline__ void sel_sort64(unsigned &k0, unsigned &w0, unsigned &k1,
-                                           unsigned &w1, int lane) {
-#pragma unroll
-    for (int k = 2; k <= 64; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j == 32) {
-                // partners i and i + 32 sit in the same lane (k == 64: ascending)
-                if (k0 > k1) {
-                    unsigned t = k0; k0 = k1; k1 = t;
-                    t = w0; w0 = w1; w1 = t;
-                }
-            } else {
-                const unsigned ok0 = __shfl_xor_sync(TT_FULL_MASK, k0, j);
-                const unsigned ow0 = __shfl_xor_sync(TT_FULL_MASK, w0, j);
-                const unsigned ok1 = __shfl_xor_sync(TT_FULL_MASK, k1, j);
-                const unsigned ow1 = __shfl_xor_sync(TT_FULL_MASK, w1, j);
-                const bool lower = (lane & j) == 0;
-                const bool up0 = (lane & k) == 0, up1 = ((lane + 32) & k) == 0;
-                // the lower element of an ascending pair keeps the smaller key
-                const bool take0 = lower == up0 ? (ok0 < k0) : (ok0 > k0);
-                const bool take1 = lower == up1 ? (ok1 < k1) : (ok1 > k1);
-                if (take0) { k0 = ok0; w0 = ow0; }
-                if (take1) { k1 = ok1; w1 = ow1; }
-            }
-        }
-    }
-}
-
-// Exact answer from a compacted list of at most 64 (key, weight) entries.
-__device__ __forceinline__ float sel_finish(const SelScratch *sc, int count,
-                                            unsigned long long below,
-                                            unsigned long long total, float fallback,
-                                            int lane) {
-    unsigned k0 = lane < count ? sc->key[lane] : 0xffffffffu;
-    unsigned w0 = lane < count ? sc->w[lane] : 0u;
-    unsigned k1 = lane + 32 < count ? sc->key[lane + 32] : 0xffffffffu;
-    unsigned w1 = lane + 32 < count ? sc->w[lane + 32] : 0u;
-    sel_sort64(k0, w0, k1, w1, lane);
-    unsigned long long c0 = w0, c1 = w1;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long t0 = __shfl_up_sync(TT_FULL_MASK, c0, d);
-        const unsigned long long t1 = __shfl_up_sync(TT_FULL_MASK, c1, d);
-        if (lane >= d) {
-            c0 += t0;
-            c1 += t1;
-        }
-    }
-    const unsigned long long half0 = __shfl_sync(TT_FULL_MASK, c0, 31);
-    c0 += below;
-    c1 += below + half0;
-    const unsigned b0 = __ballot_sync(TT_FULL_MASK, lane < count && 2ull * c0 >= total);
-    const unsigned b1 = __ballot_sync(TT_FULL_MASK, lane + 32 < count && 2ull * c1 >= total);
-    if (b0)
-        return __uint_as_float(__shfl_sync(TT_FULL_MASK, k0, __ffs(b0) - 1));
-    if (b1)
-        return __uint_as_float(__shfl_sync(TT_FULL_MASK, k1, __ffs(b1) - 1));
-    return fallback; // rounding guard: the bin's largest key
-}
-
-// Append (key, weight) of the lanes with `in` set to the list.
-__device__ __forceinline__ void sel_append(SelScratch *sc, int *count, bool in, float k,
-                                           unsigned wq, int lane) {
-    const unsigned m = __ballot_sync(TT_FULL_MASK, in);
-    if (in) {
-        const int pos = *count + __popc(m & ((1u << lane) - 1u));
-        if (pos < kSelList) {
-            sc->key[pos] = __float_as_uint(k);
-            sc->w[pos] = wq;
-        }
-    }
-    *count += __popc(m);
-}
-
-// Histogram bin of key k in [klo, klo + 256 / bs]: monotone in k, and always a
-// valid bin: keys below klo (negative samples of an image with negative
-// pixels) go to bin 0 and NaN keys convert to 0, so no input can index
-// outside the histogram.
-__device__ __forceinline__ int sel_bin(float k, float klo, float bs) {
-    return min(kSelBins - 1, max(0, (int)((k - klo) * bs)));
-}
-
-// Weighted selection over a list of keys stored in shared memory whose
-// weights are sqrt(key) (T7: the keys are the samples themselves).  The list
-// is refined in place: each round histograms [klo, khi], keeps the crossing
-// bin's keys (a strided sweep, so every write lands on an already-read slot)
-// until at most 64 remain or they are all equal.
-inline __device__ float sel_list_sqrt(float *keys, int count, float klo, float khi, float qs,
-                               unsigned long long below, unsigned long long total,
-                               SelScratch *sc, int lane) {
-    for (int level = 0; level < 16 && count > kSelList; level++) {
-        if (!(khi > klo))
-            return klo;
-        const float bs = (float)kSelBins / (khi - klo);
-        for (int i = lane; i < kSelBins; i += 32)
-            sc->hist[i] = 0u;
-        __syncwarp();
-        for (int i = lane; i < count; i += 32) {
-            const float k = keys[i];
-            atomicAdd(sc->hist + sel_bin(k, klo, bs), __float2uint_rn(sqrt_nn(k) * qs));
-        }
-        __syncwarp();
-        const int d = sel_pick_bin(sc->hist, &below, total, lane);
-        __syncwarp();
-        int nc = 0;
-        float mn = __int_as_float(0x7f800000), mx = 0.f;
-        for (int i0 = 0; i0 < count; i0 += 32) {
-            const int i = i0 + lane;
-            const float k = i < count ? keys[i] : 0.f;
-            const bool in = i < count && sel_bin(k, klo, bs) == d;
-            const unsigned m = __ballot_sync(TT_FULL_MASK, in);
-            __syncwarp();
-            if (in) {
-                keys[nc + __popc(m & ((1u << lane) - 1u))] = k;
-                mn = fminf(mn, k);
-                mx = fmaxf(mx, k);
-            }
-            nc += __popc(m);
-            __syncwarp();
-        }
-        count = nc;
-        klo = __int_as_float(warp_min(__float_as_int(mn)));
-        khi = __int_as_float(warp_max(__float_as_int(mx)));
-    }
-    if (count > kSelList)
-        return klo;
-    for (int i = lane; i < count; i += 32) {
-        sc->key[i] = __float_as_uint(keys[i]);
-        sc->w[i] = __float2uint_rn(sqrt_nn(keys[i]) * qs);
-    }
-    __syncwarp();
-    return sel_finish(sc, count, below, total, khi, lane);
-}
 
 // Fixed-point weight of a sample v: sqrt(v) (T6, T7) or v itself (P2).
 struct SqrtWeight {
@@ -220,68 +54,182 @@ struct LinearWeight {
         return __float2uint_rn(v * qs);
     }
 };
+// 2^(30 - E) for weights whose total stays below 2^E (total: their float sum).
+__device__ __forceinline__ float sel_scale(float total) {
+    const float qb = total * 1.001f;
+    const int E = ((__float_as_int(qb) >> 23) & 0xff) - 126;
+    return __int_as_float((127 + 30 - E) << 23);
+}
 
-// Interval refinement for a crossing bin that held more than 64 keys:
-// repeat histogram + compaction over [klo, khi] (the bin's key range).
-template <class KeyFn, class WFn = SqrtWeight>
-__device__ float sel_refine(const float *x, int jlo, int j0, int j1, int per, KeyFn keyfn,
-                            float qs, float klo, float khi, unsigned long long below,
-                            unsigned long long total, SelScratch *sc, int lane,
-                            WFn wfn = WFn{0.f}) {
-    if (wfn.qs == 0.f)
-        wfn.qs = qs;
+// Histogram bin of key k >= klo, bs = 256 / range: the integer that
+// (k - klo) bs rounds to, in the mantissa of 2^23, at most 255 -- monotone in
+// k.  A key below klo or NaN gives a valid bin too (255), so no input can
+// index outside the histogram; such keys carry no weight.
+constexpr unsigned kSelOne = 0x4B000000u; // 2^23
+__device__ __forceinline__ unsigned sel_bin(float k, float klo, float bs) {
+    return min((unsigned)kSelBins - 1,
+               __float_as_uint(fmaf(k - klo, bs, 8388608.f)) - kSelOne);
+}
+
+__device__ __forceinline__ void sel_clear(SelScratch *sc, int lane) {
+    uint4 *h = reinterpret_cast<uint4 *>(sc->hist);
+    h[lane] = make_uint4(0u, 0u, 0u, 0u);
+    h[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The crossing bin: the smallest bin with 2 (below + weight of the bins up to
+// it) >= total.  On entry `below` is the weight of all keys under the
+// histogram's range, on return that of all keys under the bin.  kTotal: the
+// histogram holds every weight, its sum is the total.
+struct SelPick {
+    unsigned bin, below, total;
+};
+template <bool kTotal>
+__device__ __forceinline__ SelPick sel_pick(const SelScratch *sc, unsigned below, unsigned total,
+                                            int lane) {
+    const uint4 *h4 = reinterpret_cast<const uint4 *>(sc->hist) + 2 * lane;
+    const uint4 a = h4[0], b = h4[1];
+    const unsigned h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    unsigned run = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        run += h[k];
+    unsigned inc = run;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned t = __shfl_up_sync(TT_FULL_MASK, inc, d);
+        if (lane >= d)
+            inc += t;
+    }
+    if (kTotal)
+        total = __shfl_sync(TT_FULL_MASK, inc, 31);
+    const unsigned ball = __ballot_sync(TT_FULL_MASK, 2u * (below + inc) >= total);
+    const int ln = ball ? __ffs(ball) - 1 : 31;
+    unsigned cum = below + inc - run, k = 0;
+#pragma unroll
+    for (int i = 0; i < 7; i++) { // prefix sums rise: count those that fall short
+        const bool shorter = 2u * (cum + h[i]) < total && k == (unsigned)i;
+        cum += shorter ? h[i] : 0u;
+        k += shorter;
+    }
+    SelPick p;
+    p.bin = __shfl_sync(TT_FULL_MASK, 8u * lane + k, ln);
+    p.below = __shfl_sync(TT_FULL_MASK, cum, ln);
+    p.total = total;
+    return p;
+}
+
+// Is key k in bin `bin` of a histogram from klo (bs as in sel_bin)?
+struct SelTest {
+    float klo, bs;
+    unsigned first, span;
+    __device__ __forceinline__ SelTest(float klo_, float bs_, unsigned bin)
+        : klo(klo_), bs(bs_), first(kSelOne + bin),
+          span(bin == kSelBins - 1 ? 0xffffffffu - kSelOne - bin : 0u) {}
+    __device__ __forceinline__ bool operator()(float k) const {
+        return __float_as_uint(fmaf(k - klo, bs, 8388608.f)) - first <= span;
+    }
+};
+
+// Append (key, sample) of the lanes with `in` set to the list (counted past
+// its end, never written there).
+__device__ __forceinline__ void sel_append(SelScratch *sc, int &count, bool in, float k, float v,
+                                           int lane) {
+    const unsigned m = __ballot_sync(TT_FULL_MASK, in);
+    const int pos = count + __popc(m & ((1u << lane) - 1u));
+    if (in && pos < kSelList)
+        sc->list[pos] = make_uint2(__float_as_uint(k), __float_as_uint(v));
+    count += __popc(m);
+}
+
+// The answer from a list of count <= kSelList (key, sample) entries: the
+// smallest key with 2 (below + weight of the entries up to it) >= total.
+// Keys are compared as bit patterns (the order of non-negative floats).
+template <class WFn>
+__device__ __forceinline__ float sel_answer(SelScratch *sc, int count, unsigned below,
+                                            unsigned total, WFn wfn, int lane) {
+    for (int i = lane; i < count; i += 32)
+        sc->list[i].y = wfn(__uint_as_float(sc->list[i].y));
+    __syncwarp();
+    unsigned best = 0xffffffffu, last = 0u;
+    for (int o = 0; o < count; o += 32) {
+        const bool own = o + lane < count;
+        const unsigned k = own ? sc->list[o + lane].x : 0u;
+        unsigned w = below;
+#pragma unroll 4
+        for (int i = 0; i < count; i++) {
+            const uint2 e = sc->list[i];
+            w += e.x <= k ? e.y : 0u;
+        }
+        if (own && 2u * w >= total)
+            best = min(best, k);
+        last = max(last, k);
+    }
+    best = __reduce_min_sync(TT_FULL_MASK, best);
+    last = __reduce_max_sync(TT_FULL_MASK, last); // never needed: the bin holds the crossing
+    return __uint_as_float(best == 0xffffffffu ? last : best);
+}
+
+// Refinement of a crossing bin that held more than kSelList entries: `in` tells
+// its members among the line's elements e in [0, cnt) (samples xb[e], keys
+// keyfn(e, v)).  Each level finds the members' key range and histograms it.
+template <class KeyFn, class WFn>
+__device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, WFn wfn,
+                                         SelTest in, SelPick p, SelScratch *sc, int lane) {
+    float klo = 0.f, khi = 0.f;
     for (int level = 0; level < 8; level++) {
+        // key range of the members (level > 0: of the last bin's, inside the
+        // last range)
+        float mn = __int_as_float(0x7f800000), mx = 0.f;
+        for (int e = lane; e < cnt; e += 32) {
+            const float v = xb[e], k = keyfn(e, v);
+            if (in(k) && (level == 0 || (k >= klo && k <= khi))) {
+                mn = fminf(mn, k);
+                mx = fmaxf(mx, k);
+            }
+        }
+        klo = __int_as_float(warp_min(__float_as_int(mn)));
+        khi = __int_as_float(warp_max(__float_as_int(mx)));
         if (!(khi > klo))
             return klo;
         const float bs = (float)kSelBins / (khi - klo);
-        for (int i = lane; i < kSelBins; i += 32)
-            sc->hist[i] = 0u;
         __syncwarp();
-        for (int i = 0; i < per; i++) { // warp-uniform trip count
-            const int j = j0 + i;
-            const float v = j < j1 ? x[j - jlo] : 0.f;
-            const float k = keyfn(j, v);
-            if (j < j1 && k >= klo && k <= khi)
+        sel_clear(sc, lane);
+        __syncwarp();
+        for (int e = lane; e < cnt; e += 32) {
+            const float v = xb[e], k = keyfn(e, v);
+            if (k >= klo && k <= khi)
                 atomicAdd(sc->hist + sel_bin(k, klo, bs), wfn(v));
         }
         __syncwarp();
-        const int d = sel_pick_bin(sc->hist, &below, total, lane);
+        p = sel_pick<false>(sc, p.below, p.total, lane);
+        in = SelTest(klo, bs, p.bin);
         __syncwarp();
         int count = 0;
-        float bmin = __int_as_float(0x7f800000), bmax = 0.f;
-        for (int i = 0; i < per; i++) {
-            const int j = j0 + i;
-            const float v = j < j1 ? x[j - jlo] : 0.f;
-            const float k = keyfn(j, v);
-            const bool in = j < j1 && k >= klo && k <= khi && sel_bin(k, klo, bs) == d;
-            const unsigned wq = in ? wfn(v) : 0u;
-            bmin = in ? fminf(bmin, k) : bmin;
-            bmax = in ? fmaxf(bmax, k) : bmax;
-            sel_append(sc, &count, in, k, wq, lane);
+        for (int e0 = 0; e0 < cnt; e0 += 32) {
+            const int e = e0 + lane;
+            const float v = e < cnt ? xb[e] : 0.f, k = keyfn(e, v);
+            sel_append(sc, count, e < cnt && k >= klo && k <= khi && in(k), k, v, lane);
         }
-        bmin = __int_as_float(warp_min(__float_as_int(bmin)));
-        bmax = __int_as_float(warp_max(__float_as_int(bmax)));
         __syncwarp();
         if (count <= kSelList)
-            return sel_finish(sc, count, below, total, bmax, lane);
-        klo = bmin;
-        khi = bmax;
-        __syncwarp();
+            return sel_answer(sc, count, p.below, p.total, wfn, lane);
     }
     return klo;
 }
 
 // T6 and T7 of one line (c++/src/functionals.cpp:226-276).  T6: keys
 // r1 * x[m2 + r1], r1 in [0, N - m2); T7: keys x[m1 ..]; both weighted by
-// sqrt(x).  One histogram pass serves both (a chunked sweep: far-apart
-// elements in flight, so fewer atomic collisions); T6 then compacts its bin
-// into a 64-entry list, and T7 -- last, because it overwrites the line --
-// compacts its bin in place and refines on that list.  xmax and qtot (the
-// line's largest sample and sum of square roots) bound every key and weight
-// total, so no separate range pass is needed.
-inline __device__ void select_t67(float *x, int jlo, int jhi, int m1, int m2, bool want6,
-                           bool want7, float xmax, float qtot, SelScratch *s6, SelScratch *s7,
-                           int lane, float *r6, float *r7) {
+// sqrt(x).  Elements are the line's stored rows at x[row - jlo]; every other
+// row is a zero sample (key 0, weight 0), which cannot move the crossing
+// unless all weights are zero, in which case the reference returns its
+// smallest key, 0.  One histogram pass and one collecting pass serve both (a
+// chunked sweep: far-apart elements in flight, so fewer atomic collisions).
+// xmax and qtot (the line's largest sample and sum of square roots) bound
+// every key and weight total, so no separate range pass is needed.
+inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int m2, bool want6,
+                                  bool want7, float xmax, float qtot, SelScratch *s6,
+                                  SelScratch *s7, int lane, float *r6, float *r7) {
     *r6 = 0.f;
     *r7 = 0.f;
     const int b7 = max(m1, jlo), b6 = max(m2, jlo);
@@ -290,107 +238,98 @@ inline __device__ void select_t67(float *x, int jlo, int jhi, int m1, int m2, bo
     if (cnt <= 0 || !(xmax > 0.f) || !(qtot > 0.f))
         return;
     const int per = ((cnt + 31) >> 5) | 1; // odd: conflict-free chunks
-    const int j0 = min(b + lane * per, jhi), j1 = min(j0 + per, jhi);
-    // u32 fixed-point weights: q = 2^(30 - E), every weight total < 2^E
-    const float qb = qtot * 1.001f;
-    const int E = ((__float_as_int(qb) >> 23) & 0xff) - 126;
-    const float qs = __int_as_float((127 + 30 - E) << 23);
+    const SqrtWeight wfn{sel_scale(qtot)};
     const float k6max = __fmul_rn((float)max(jhi - 1 - m2, 0), xmax);
     want6 = want6 && k6max > 0.f; // otherwise every T6 key is 0
     const float bs7 = (float)kSelBins / xmax, bs6 = want6 ? (float)kSelBins / k6max : 0.f;
-    auto key6 = [b6, m2](int j, float v) { return j >= b6 ? __fmul_rn((float)(j - m2), v) : -1.f; };
+    // element e of [0, cnt) is row b + e; this lane's are e0 .. e0 + mine - 1,
+    // of which T7 takes those from i = f7 on and T6 those from f6
+    const float *xb = x + (b - jlo);
+    const int e0 = lane * per, mine = min(max(cnt - e0, 0), per);
+    const int f7 = want7 ? b7 - b - e0 : per, f6 = want6 ? b6 - b - e0 : per;
+    const float r0 = (float)(b + e0 - m2); // T6's factor of the lane's first element
 
-    for (int i = lane; i < kSelBins; i += 32) {
-        s6->hist[i] = 0u;
-        s7->hist[i] = 0u;
-    }
+    sel_clear(s6, lane);
+    sel_clear(s7, lane);
     __syncwarp();
-    unsigned l6 = 0, l7 = 0, l7max = 0;
+    unsigned l7max = 0;
+    float rf = r0; // exact: integers below 2^24
     // a warp-uniform trip count (per), lanes past their chunk predicated off
-    for (int i0 = 0; i0 < per; i0 += 4) {
+    for (int i0 = 0; i0 < per; i0 += 4, rf += 4.f) {
         float vb[4]; // four loads in flight before the atomics
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int j = j0 + i0 + u;
-            vb[u] = j < j1 ? x[j - jlo] : 0.f;
-        }
+        for (int u = 0; u < 4; u++)
+            vb[u] = i0 + u < mine ? xb[e0 + i0 + u] : 0.f;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const int j = j0 + i0 + u;
+            const int i = i0 + u;
             const float v = vb[u];
-            const unsigned wq = __float2uint_rn(sqrt_nn(v) * qs);
-            const bool in7 = want7 && j >= b7 && j < j1, in6 = want6 && j >= b6 && j < j1;
-            l7 += in7 ? wq : 0u;
-            l7max += in7 && v == xmax ? wq : 0u;
-            l6 += in6 ? wq : 0u;
-            if (in7)
+            const unsigned wq = wfn(v); // 0 past the chunk
+            l7max += v == xmax && i >= f7 ? wq : 0u;
+            if (wq && i >= f7)
                 atomicAdd(s7->hist + sel_bin(v, 0.f, bs7), wq);
-            if (in6)
-                atomicAdd(s6->hist + sel_bin(key6(j, v), 0.f, bs6), wq);
+            if (wq && i >= f6)
+                atomicAdd(s6->hist + sel_bin(__fmul_rn(rf + (float)u, v), 0.f, bs6), wq);
         }
-    }
-    const unsigned long long W7 = __reduce_add_sync(TT_FULL_MASK, l7);
-    const unsigned long long W6 = __reduce_add_sync(TT_FULL_MASK, l6);
-    // Saturated lines (samples clipped at the image's maximum) put the
-    // crossing on the largest key: when the keys below the maximum weigh less
-    // than half the total, 2 W(< xmax) < W, the answer is xmax -- exact in
-    // the fixed-point weights, no compaction or refinement needed.
-    const unsigned long long W7max = __reduce_add_sync(TT_FULL_MASK, l7max);
-    if (want7 && W7max > 0 && 2ull * (W7 - W7max) < W7) {
-        *r7 = xmax;
-        want7 = false;
     }
     __syncwarp();
-
-    if (want6) {
-        unsigned long long below = 0;
-        const int d = sel_pick_bin(s6->hist, &below, W6, lane);
-        __syncwarp();
-        int c = 0;
-        float mn = __int_as_float(0x7f800000), mx = 0.f;
-        for (int i = 0; i < per; i++) {
-            const int j = j0 + i;
-            const float v = j < j1 ? x[j - jlo] : 0.f;
-            const float k = key6(j, v);
-            const bool in = j < j1 && j >= b6 && sel_bin(k, 0.f, bs6) == d;
-            const unsigned wq = in ? __float2uint_rn(sqrt_nn(v) * qs) : 0u;
-            mn = in ? fminf(mn, k) : mn;
-            mx = in ? fmaxf(mx, k) : mx;
-            sel_append(s6, &c, in, k, wq, lane);
-        }
-        mn = __int_as_float(warp_min(__float_as_int(mn)));
-        mx = __int_as_float(warp_max(__float_as_int(mx)));
-        __syncwarp();
-        if (c <= kSelList)
-            *r6 = sel_finish(s6, c, below, W6, mx, lane);
-        else
-            *r6 = sel_refine(x, jlo, j0, j1, per, key6, qs, mn, mx, below, W6, s6, lane);
-    }
-
+    SelPick p7{0u, 0u, 0u}, p6{0u, 0u, 0u};
     if (want7) {
-        unsigned long long below = 0;
-        const int d = sel_pick_bin(s7->hist, &below, W7, lane);
-        __syncwarp();
-        // in-place compaction: the write index never passes the read index
-        int c = 0;
-        float mn = __int_as_float(0x7f800000), mx = 0.f;
-        for (int js = b7; js < jhi; js += 32) {
-            const int j = js + lane;
-            const float v = j < jhi ? x[j - jlo] : 0.f;
-            const bool in = j < jhi && sel_bin(v, 0.f, bs7) == d;
-            const unsigned m = __ballot_sync(TT_FULL_MASK, in);
-            __syncwarp();
-            if (in) {
-                x[c + __popc(m & ((1u << lane) - 1u))] = v;
-                mn = fminf(mn, v);
-                mx = fmaxf(mx, v);
-            }
-            c += __popc(m);
-            __syncwarp();
+        p7 = sel_pick<true>(s7, 0u, 0u, lane);
+        // Saturated lines (samples clipped at the image's maximum) put the
+        // crossing on the largest key: when the keys below the maximum weigh
+        // less than half the total, 2 W(< xmax) < W, the answer is xmax.
+        const unsigned wmax = __reduce_add_sync(TT_FULL_MASK, l7max);
+        if (wmax > 0 && 2u * (p7.total - wmax) < p7.total) {
+            *r7 = xmax;
+            want7 = false;
         }
-        mn = __int_as_float(warp_min(__float_as_int(mn)));
-        mx = __int_as_float(warp_max(__float_as_int(mx)));
-        *r7 = sel_list_sqrt(x, c, mn, mx, qs, below, W7, s7, lane);
+    }
+    if (want6)
+        p6 = sel_pick<true>(s6, 0u, 0u, lane);
+    if (!want6 && !want7)
+        return;
+    __syncwarp(); // both histograms are read: the lists take their place
+    const SelTest in7(0.f, bs7, p7.bin), in6(0.f, bs6, p6.bin);
+    int c6 = 0, c7 = 0;
+    rf = r0;
+    for (int i0 = 0; i0 < per; i0 += 4, rf += 4.f) {
+        float vb[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            vb[u] = i0 + u < mine ? xb[e0 + i0 + u] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = i0 + u;
+            const float v = vb[u], k6 = __fmul_rn(rf + (float)u, v);
+            const bool a7 = want7 && i >= f7 && i < mine && in7(v);
+            const bool a6 = want6 && i >= f6 && i < mine && in6(k6);
+            if (__any_sync(TT_FULL_MASK, a7 || a6)) {
+                sel_append(s7, c7, a7, v, v, lane);
+                sel_append(s6, c6, a6, k6, v, lane);
+            }
+        }
+    }
+    __syncwarp();
+    if (want7) {
+        if (c7 <= kSelList) {
+            *r7 = sel_answer(s7, c7, p7.below, p7.total, wfn, lane);
+        } else {
+            const int o7 = b7 - b;
+            *r7 = sel_refine(xb + o7, cnt - o7, [](int, float v) { return v; }, wfn, in7, p7, s7,
+                             lane);
+        }
+    }
+    if (want6) {
+        if (c6 <= kSelList) {
+            *r6 = sel_answer(s6, c6, p6.below, p6.total, wfn, lane);
+        } else {
+            const int o6 = b6 - b;
+            const float rb = (float)(b6 - m2);
+            *r6 = sel_refine(xb + o6, cnt - o6,
+                             [rb](int e, float v) { return __fmul_rn(rb + (float)e, v); }, wfn,
+                             in6, p6, s6, lane);
+        }
     }
 }
 
@@ -400,61 +339,50 @@ inline __device__ void select_t67(float *x, int jlo, int jhi, int m1, int m2, bo
 // column in shared memory, n values, xmax their maximum, xsum their sum (a
 // bound for the fixed-point scale).  One warp.
 inline __device__ float select_p2(const float *x, int n, float xmax, float xsum, SelScratch *sc,
-                           int lane) {
+                                  int lane) {
     if (n <= 0)
         return 0.f;
     if (!(xmax > 0.f) || !(xsum > 0.f))
         return 0.f; // all zero: the first sorted value
     const int per = ((n + 31) >> 5) | 1;
-    const int j0 = min(lane * per, n), j1 = min(j0 + per, n);
-    const float qb = xsum * 1.001f;
-    const int E = ((__float_as_int(qb) >> 23) & 0xff) - 126;
-    const float qs = __int_as_float((127 + 30 - E) << 23);
-    const LinearWeight wfn{qs};
+    const int j0 = lane * per, mine = min(max(n - j0, 0), per);
+    const LinearWeight wfn{sel_scale(xsum)};
     const float bs = (float)kSelBins / xmax;
-    for (int i = lane; i < kSelBins; i += 32)
-        sc->hist[i] = 0u;
+    sel_clear(sc, lane);
     __syncwarp();
-    unsigned lw = 0;
     for (int i0 = 0; i0 < per; i0 += 4) { // warp-uniform trip count
         float vb[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int j = j0 + i0 + u;
-            vb[u] = j < j1 ? x[j] : 0.f;
-        }
+        for (int u = 0; u < 4; u++)
+            vb[u] = i0 + u < mine ? x[j0 + i0 + u] : 0.f;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const bool in = j0 + i0 + u < j1;
             const unsigned wq = wfn(vb[u]);
-            lw += in ? wq : 0u;
-            if (in)
+            if (wq)
                 atomicAdd(sc->hist + sel_bin(vb[u], 0.f, bs), wq);
         }
     }
-    const unsigned long long W = __reduce_add_sync(TT_FULL_MASK, lw);
     __syncwarp();
-    unsigned long long below = 0;
-    const int d = sel_pick_bin(sc->hist, &below, W, lane);
+    const SelPick p = sel_pick<true>(sc, 0u, 0u, lane);
     __syncwarp();
+    const SelTest in(0.f, bs, p.bin);
     int c = 0;
-    float mn = __int_as_float(0x7f800000), mx = 0.f;
-    for (int i = 0; i < per; i++) {
-        const int j = j0 + i;
-        const float k = j < j1 ? x[j] : 0.f;
-        const bool in = j < j1 && sel_bin(k, 0.f, bs) == d;
-        const unsigned wq = in ? wfn(k) : 0u;
-        mn = in ? fminf(mn, k) : mn;
-        mx = in ? fmaxf(mx, k) : mx;
-        sel_append(sc, &c, in, k, wq, lane);
+    for (int i0 = 0; i0 < per; i0 += 4) {
+        float vb[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            vb[u] = i0 + u < mine ? x[j0 + i0 + u] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool a = i0 + u < mine && in(vb[u]);
+            if (__any_sync(TT_FULL_MASK, a))
+                sel_append(sc, c, a, vb[u], vb[u], lane);
+        }
     }
-    mn = __int_as_float(warp_min(__float_as_int(mn)));
-    mx = __int_as_float(warp_max(__float_as_int(mx)));
     __syncwarp();
     if (c <= kSelList)
-        return sel_finish(sc, c, below, W, mx, lane);
-    auto key = [](int, float v) { return v; };
-    return sel_refine(x, 0, j0, j1, per, key, qs, mn, mx, below, W, sc, lane, wfn);
+        return sel_answer(sc, c, p.below, p.total, wfn, lane);
+    return sel_refine(x, n, [](int, float v) { return v; }, wfn, in, p, sc, lane);
 }
 
 } // namespace tt
