@@ -21,10 +21,9 @@
 // element as it needs -- bins by one multiply-add into the mantissa of 2^23,
 // weights (a square root each) only in the histogram pass and for the few
 // collected entries -- and the fixed work per line.  The collected list takes
-// the histogram's place in shared memory.  1024^2 x 360 angles, T0-T7: 2.55 ms,
-// of which T6 and T7 1.17 (3.21 and 1.79 with the bins recomputed by
-// conversions and the weights in both passes, 64-bit scans and a 64-entry
-// bitonic sort).
+// the histogram's place in shared memory.  1024^2 x 360 angles, T0-T7: 2.55 ms
+// (3.21 with the bins recomputed by conversions and the weights in both
+// passes, 64-bit scans and a 64-entry bitonic sort).
 #pragma once
 
 #include "tt_common.cuh"
@@ -44,8 +43,9 @@ struct __align__(16) SelScratch {
 // Fixed-point weight of a sample v: sqrt(v) (T6, T7) or v itself (P2).
 struct SqrtWeight {
     float qs;
+    bool odd; // the line holds samples sqrt_pos does not take (warp-uniform)
     __device__ __forceinline__ unsigned operator()(float v) const {
-        return __float2uint_rn(sqrt_nn(v) * qs);
+        return __float2uint_rn((odd ? sqrt_nn(v) : sqrt_pos(v)) * qs);
     }
 };
 struct LinearWeight {
@@ -226,10 +226,12 @@ __device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, 
 // smallest key, 0.  One histogram pass and one collecting pass serve both (a
 // chunked sweep: far-apart elements in flight, so fewer atomic collisions).
 // xmax and qtot (the line's largest sample and sum of square roots) bound
-// every key and weight total, so no separate range pass is needed.
+// every key and weight total, so no separate range pass is needed; odd: some
+// sample is none sqrt_pos takes.
 inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int m2, bool want6,
-                                  bool want7, float xmax, float qtot, SelScratch *s6,
-                                  SelScratch *s7, int lane, float *r6, float *r7) {
+                                  bool want7, float xmax, float qtot, bool odd,
+                                  SelScratch *s6, SelScratch *s7, int lane, float *r6,
+                                  float *r7) {
     *r6 = 0.f;
     *r7 = 0.f;
     const int b7 = max(m1, jlo), b6 = max(m2, jlo);
@@ -238,7 +240,7 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
     if (cnt <= 0 || !(xmax > 0.f) || !(qtot > 0.f))
         return;
     const int per = ((cnt + 31) >> 5) | 1; // odd: conflict-free chunks
-    const SqrtWeight wfn{sel_scale(qtot)};
+    const SqrtWeight wfn{sel_scale(qtot), odd};
     const float k6max = __fmul_rn((float)max(jhi - 1 - m2, 0), xmax);
     want6 = want6 && k6max > 0.f; // otherwise every T6 key is 0
     const float bs7 = (float)kSelBins / xmax, bs6 = want6 ? (float)kSelBins / k6max : 0.f;

@@ -85,9 +85,53 @@ __device__ __forceinline__ int resolve_median(int found, float total, int jlo,
     return n - 1;
 }
 
+// The square root of a sample; odd: it may be one sqrt_pos does not take.
+__device__ __forceinline__ float root(float v, bool odd) {
+    return odd ? sqrt_nn(v) : sqrt_pos(v);
+}
 template <bool kSqrt>
-__device__ __forceinline__ float elem(const float *x, int i) {
-    return kSqrt ? sqrt_nn(x[i]) : x[i];
+__device__ __forceinline__ float elem(const float *x, int i, bool odd) {
+    return kSqrt ? root(x[i], odd) : x[i];
+}
+
+// The sums of one lane's chunk of C samples in storage order, plain and (kRoot)
+// of the square roots, its largest sample (kMax) and what the samples are:
+// odd -- some sample of the warp is none that sqrt_pos takes -- and neg -- some
+// sample of it is negative.  Odd samples are rare (no 8-bit image has them),
+// so the common pass only watches for them and the warp that meets one
+// sums again with the general square root.  1024^2 x 360 angles, T0-T7: 2.25
+// ms (2.55 with the general root, its range tests and branches throughout);
+// 4096^2 x 720: 84.9 from 105.7 ms; 389 x 640 x 360, T0-T5: 278 from 318 us.
+struct ChunkSums {
+    float tot = 0.f, totq = 0.f, top = 0.f;
+    bool odd = false, neg = false;
+};
+template <bool kRoot>
+__device__ __forceinline__ ChunkSums chunk_sums(const float *x, int C) {
+    ChunkSums r;
+    RootRange range;
+#pragma unroll 4
+    for (int k = 0; k < C; k++) {
+        const float v = x[k];
+        r.tot += v;
+        range.add(v);
+        if (kRoot)
+            r.totq += sqrt_pos(v);
+    }
+    r.top = __uint_as_float(range.top);
+    r.odd = __any_sync(TT_FULL_MASK, range.odd());
+    if (r.odd) {
+        r.totq = r.top = 0.f;
+        for (int k = 0; k < C; k++) {
+            const float v = x[k];
+            r.neg |= v < 0.f;
+            r.top = fmaxf(r.top, v);
+            if (kRoot)
+                r.totq += sqrt_nn(v);
+        }
+        r.neg = __any_sync(TT_FULL_MASK, r.neg);
+    }
+    return r;
 }
 
 // First element i (of the chunked line) with 2 * prefix_i >= total, given the
@@ -95,7 +139,8 @@ __device__ __forceinline__ float elem(const float *x, int i) {
 // crosses and scans that chunk cooperatively (continuing into the next chunk
 // if rounding put the crossing there).  Valid for non-negative data.
 template <bool kSqrt>
-__device__ int find_crossing(const float *x, int C, float inc, float exc, float total, int lane) {
+__device__ int find_crossing(const float *x, int C, float inc, float exc, float total, bool odd,
+                             int lane) {
     const unsigned ball = __ballot_sync(TT_FULL_MASK, 2.f * inc >= total);
     if (!ball)
         return INT_MAX;
@@ -103,7 +148,7 @@ __device__ int find_crossing(const float *x, int C, float inc, float exc, float 
         float basev = __shfl_sync(TT_FULL_MASK, exc, ln);
         for (int t0 = 0; t0 < C; t0 += 32) {
             const int t = t0 + lane;
-            const float v = t < C ? elem<kSqrt>(x, ln * C + t) : 0.f;
+            const float v = t < C ? elem<kSqrt>(x, ln * C + t, odd) : 0.f;
             const float p = warp_incl_scan(v, lane) + basev;
             const unsigned b = __ballot_sync(TT_FULL_MASK, t < C && 2.f * p >= total);
             if (b)
@@ -241,24 +286,13 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     const bool need_sq = need_m2 || (need & (1u << 7)); // sum of sqrt(x) wanted
     const int base = lane * C;
 
-    float tot = 0.f, totq = 0.f, lmax = 0.f;
-    bool neg = false;
-#pragma unroll 4
-    for (int k = 0; k < C; k++) {
-        const float v = x[base + k];
-        tot += v;
-        neg |= v < 0.f;
-        if (kSel)
-            lmax = fmaxf(lmax, v);
-        if (need_sq)
-            totq += sqrt_nn(v);
-    }
-    const float inc = warp_incl_scan(tot, lane);
+    const ChunkSums cs = need_sq ? chunk_sums<true>(x + base, C) : chunk_sums<false>(x + base, C);
+    const float inc = warp_incl_scan(cs.tot, lane);
     const float S = __shfl_sync(TT_FULL_MASK, inc, 31);
     float exc = __shfl_up_sync(TT_FULL_MASK, inc, 1);
     float Q = 0.f, incq = 0.f, excq = 0.f;
     if (need_sq) {
-        incq = warp_incl_scan(totq, lane);
+        incq = warp_incl_scan(cs.totq, lane);
         Q = __shfl_sync(TT_FULL_MASK, incq, 31);
         excq = __shfl_up_sync(TT_FULL_MASK, incq, 1);
     }
@@ -266,16 +300,15 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
         exc = 0.f;
         excq = 0.f;
     }
-    const bool any_neg = __any_sync(TT_FULL_MASK, neg);
 
     int m1 = 0, m2 = 0;
     if (need_m1) {
-        const int f = any_neg ? find_crossing_walk(x, C, exc, S, lane)
-                              : find_crossing<false>(x, C, inc, exc, S, lane);
+        const int f = cs.neg ? find_crossing_walk(x, C, exc, S, lane)
+                              : find_crossing<false>(x, C, inc, exc, S, false, lane);
         m1 = resolve_median(f, S, jlo, jhi, len, n);
     }
     if (need_m2)
-        m2 = resolve_median(find_crossing<true>(x, C, incq, excq, Q, lane), Q, jlo, jhi, len, n);
+        m2 = resolve_median(find_crossing<true>(x, C, incq, excq, Q, cs.odd, lane), Q, jlo, jhi, len, n);
 
     float r1v = 0.f, r2v = 0.f;
     if (need & ((1u << 1) | (1u << 2))) {
@@ -330,9 +363,9 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     float r6v = 0.f, r7v = 0.f;
     if (kSel) {
         SelScratch *scr = reinterpret_cast<SelScratch *>(sm + L * stride) + 2 * warp;
-        const float xmax = __int_as_float(warp_max(__float_as_int(lmax)));
+        const float xmax = __int_as_float(warp_max(__float_as_int(cs.top)));
         // T6: keys r1 * x[m2 + r1], r1 in [0, N - m2); T7: keys x[m1 ..]
-        select_t67(x, jlo, jhi, m1, m2, need & (1u << 6), need & (1u << 7), xmax, Q, scr,
+        select_t67(x, jlo, jhi, m1, m2, need & (1u << 6), need & (1u << 7), xmax, Q, cs.odd, scr,
                    scr + 1, lane, &r6v, &r7v);
     }
 
@@ -500,8 +533,8 @@ template <int SW> __device__ __forceinline__ unsigned seg_ballot(bool p, int s) 
 
 // find_crossing per segment; every lane runs the same (warp-uniform) loops.
 template <bool kSqrt, int SW>
-__device__ int seg_find_crossing(const float *x, int C, float inc, float exc, float total, int s,
-                                 int sub) {
+__device__ int seg_find_crossing(const float *x, int C, float inc, float exc, float total,
+                                 bool odd, int s, int sub) {
     const unsigned ball = seg_ballot<SW>(2.f * inc >= total, s);
     int ln = ball ? __ffs(ball) - 1 : SW;
     int found = INT_MAX;
@@ -511,7 +544,7 @@ __device__ int seg_find_crossing(const float *x, int C, float inc, float exc, fl
         for (int t0 = 0; t0 < C; t0 += SW) {
             const int t = t0 + sub;
             const bool in = active && t < C;
-            const float v = in ? elem<kSqrt>(x, ln * C + t) : 0.f;
+            const float v = in ? elem<kSqrt>(x, ln * C + t, odd) : 0.f;
             const float p = seg_incl_scan<SW>(v, sub) + basev;
             const unsigned b = seg_ballot<SW>(in && 2.f * p >= total, s);
             if (active && b) {
@@ -531,8 +564,8 @@ __device__ int seg_find_crossing(const float *x, int C, float inc, float exc, fl
 // exc2); the same result as two seg_find_crossing calls, in one loop.
 template <int SW>
 __device__ void seg_find_crossing2(const float *x, int C, float inc1, float exc1, float tot1,
-                                   float inc2, float exc2, float tot2, int s, int sub, int &f1,
-                                   int &f2) {
+                                   float inc2, float exc2, float tot2, bool odd, int s, int sub,
+                                   int &f1, int &f2) {
     const unsigned b1 = seg_ballot<SW>(2.f * inc1 >= tot1, s);
     const unsigned b2 = seg_ballot<SW>(2.f * inc2 >= tot2, s);
     int ln1 = b1 ? __ffs(b1) - 1 : SW, ln2 = b2 ? __ffs(b2) - 1 : SW;
@@ -546,7 +579,7 @@ __device__ void seg_find_crossing2(const float *x, int C, float inc1, float exc1
             const int t = t0 + sub;
             const bool in1 = a1 && t < C, in2 = a2 && t < C;
             const float v1 = in1 ? x[ln1 * C + t] : 0.f;
-            const float v2 = in2 ? sqrt_nn(x[ln2 * C + t]) : 0.f;
+            const float v2 = in2 ? root(x[ln2 * C + t], odd) : 0.f;
             const float p1 = seg_incl_scan<SW>(v1, sub) + base1;
             const float p2 = seg_incl_scan<SW>(v2, sub) + base2;
             const unsigned c1 = seg_ballot<SW>(in1 && 2.f * p1 >= tot1, s);
@@ -704,21 +737,13 @@ __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_
     const bool need_m1 = need & ((1u << 1) | (1u << 2));
     const bool need_m2 = need & ((1u << 3) | (1u << 4) | (1u << 5));
     const int base = sub * C;
-    float tot = 0.f, totq = 0.f;
-    bool neg = false;
-    for (int k = 0; k < C; k++) {
-        const float v = x[base + k];
-        tot += v;
-        neg |= v < 0.f;
-        if (need_m2)
-            totq += sqrt_nn(v);
-    }
-    const float inc = seg_incl_scan<SW>(tot, sub);
+    const ChunkSums cs = need_m2 ? chunk_sums<true>(x + base, C) : chunk_sums<false>(x + base, C);
+    const float inc = seg_incl_scan<SW>(cs.tot, sub);
     const float S = __shfl_sync(TT_FULL_MASK, inc, s * SW + SW - 1);
     float exc = __shfl_up_sync(TT_FULL_MASK, inc, 1, SW);
     float Q = 0.f, incq = 0.f, excq = 0.f;
     if (need_m2) {
-        incq = seg_incl_scan<SW>(totq, sub);
+        incq = seg_incl_scan<SW>(cs.totq, sub);
         Q = __shfl_sync(TT_FULL_MASK, incq, s * SW + SW - 1);
         excq = __shfl_up_sync(TT_FULL_MASK, incq, 1, SW);
     }
@@ -726,21 +751,20 @@ __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_
         exc = 0.f;
         excq = 0.f;
     }
-    const bool any_neg = __any_sync(TT_FULL_MASK, neg);
     int m1 = 0, m2 = 0;
-    if (need_m1 && need_m2 && !any_neg) {
+    if (need_m1 && need_m2 && !cs.neg) {
         int f1, f2;
-        seg_find_crossing2<SW>(x, C, inc, exc, S, incq, excq, Q, s, sub, f1, f2);
+        seg_find_crossing2<SW>(x, C, inc, exc, S, incq, excq, Q, cs.odd, s, sub, f1, f2);
         m1 = resolve_median(f1, S, jlo, jhi, len, n);
         m2 = resolve_median(f2, Q, jlo, jhi, len, n);
     } else {
         if (need_m1) {
-            const int f = any_neg ? seg_walk<SW>(x, C, exc, S, sub)
-                                  : seg_find_crossing<false, SW>(x, C, inc, exc, S, s, sub);
+            const int f = cs.neg ? seg_walk<SW>(x, C, exc, S, sub)
+                                  : seg_find_crossing<false, SW>(x, C, inc, exc, S, false, s, sub);
             m1 = resolve_median(f, S, jlo, jhi, len, n);
         }
         if (need_m2)
-            m2 = resolve_median(seg_find_crossing<true, SW>(x, C, incq, excq, Q, s, sub), Q, jlo,
+            m2 = resolve_median(seg_find_crossing<true, SW>(x, C, incq, excq, Q, cs.odd, s, sub), Q, jlo,
                                 jhi, len, n);
     }
 
