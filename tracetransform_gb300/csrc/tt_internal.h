@@ -37,6 +37,7 @@ struct SinoArgs {
     unsigned need;      // bit f set when T-functional f is requested
     int stride;         // floats per line in shared memory
     bool interior;      // the texture region lies >= 2 texels inside the frame
+    float neg_zero = -0.f; // an addend no compiler pass sees through (sample_line)
 };
 
 // Does a texture region of rows x cols at (row_off, col_off) lie at least two
@@ -279,6 +280,7 @@ struct BatchSinoArgs {
     unsigned need;
     int stride;              // floats per line buffer (for the largest n)
     bool all_interior;       // every image passes interior_source
+    float neg_zero = -0.f;   // as in SinoArgs
 };
 
 int sino_lines_per_block(int n, unsigned need);

@@ -10,14 +10,13 @@
 // Sampling.  The source region sits in a block-linear CUDA array read through
 // a texture object in border mode (texels outside the region read 0, which
 // is exactly the reference's zero padding).  One 2x2 gather (tld4) fetches
-// the bilinear stencil; coordinates and weights are then combined in the
-// reference's order with scalar round-to-nearest operations, so every
-// rotated sample is bit-identical to rotate()/interpolate()
+// the bilinear stencil; coordinates and weights are combined in the
+// reference's order, every operation rounded on its own, so every rotated
+// sample is bit-identical to rotate()/interpolate()
 // (c++/src/auxiliary.cpp:182-196, 223-255): the host rounds cos/sin as the
-// reference does and no multiply-add is fused.  (Packed f32x2 multiply + add
-// measured fused on this part, so they are not used here.)  Each thread keeps
-// four gathers in flight.  Only rows whose stencil can touch the image are
-// sampled; all others are exact zeros in the reference too.
+// reference does and no multiply-add is fused (see sample_line).  Each thread
+// keeps four gathers in flight.  Only rows whose stencil can touch the image
+// are sampled; all others are exact zeros in the reference too.
 //
 // Reductions run in warp order rather than the reference's sequential order,
 // so sums agree to rounding and a weighted median can move by one row where
@@ -172,11 +171,46 @@ __device__ int find_crossing_walk(const float *x, int C, float exc, float total,
     return warp_min(f);
 }
 
+// One lane's share of T3-T5's complex sums over q = q0, q0 + STEP, ... < q1 of
+// the tables' kernels times x[q].  All three at once (the usual call) without a
+// test per term; one 32-bit offset serves the three tables.
+template <int STEP>
+__device__ __forceinline__ void tail345(const float2 *tab, int n, const float *x, int q0, int q1,
+                                        bool w3, bool w4, bool w5, float &re3, float &im3,
+                                        float &re4, float &im4, float &re5, float &im5) {
+    const float2 *tab3 = tab, *tab4 = tab + n, *tab5 = tab + 2 * n;
+    auto term = [](const float2 *t, unsigned q, float v, float &re, float &im) {
+        const float2 w = __ldg(t + q);
+        re = fmaf(w.x, v, re);
+        im = fmaf(w.y, v, im);
+    };
+    if (w3 && w4 && w5) {
+#pragma unroll 2
+        for (int q = q0; q < q1; q += STEP) {
+            const float v = x[q];
+            term(tab3, (unsigned)q, v, re3, im3);
+            term(tab4, (unsigned)q, v, re4, im4);
+            term(tab5, (unsigned)q, v, re5, im5);
+        }
+        return;
+    }
+    for (int q = q0; q < q1; q += STEP) {
+        const float v = x[q];
+        if (w3)
+            term(tab3, (unsigned)q, v, re3, im3);
+        if (w4)
+            term(tab4, (unsigned)q, v, re4, im4);
+        if (w5)
+            term(tab5, (unsigned)q, v, re5, im5);
+    }
+}
+
 // One CTA's unit of work: L adjacent lines (columns col0 ..) of one angle of
 // one image.
 struct BlockJob {
     cudaTextureObject_t tex;
     float tu, tv;     // texel coordinate = frame coordinate + (tu, tv)
+    float neg_zero;   // -0 (see sample_line)
     int n, col0, angle;
     float c, s;       // cos(-theta), sin(-theta) as the host rounded them
     int roff, coff, rr, rc; // support region inside the frame
@@ -185,6 +219,121 @@ struct BlockJob {
     int32_t *medians;       // optional, same shape
     size_t plane;           // n_angles * n
 };
+
+// ---- sampling ------------------------------------------------------------------
+
+// Two floats in one 64-bit register pair, as the packed f32x2 operations take
+// them: one issue slot for both halves.
+using pair2 = unsigned long long;
+__device__ __forceinline__ pair2 pack2(float lo, float hi) {
+    pair2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(pair2 a) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(a));
+    return d;
+}
+__device__ __forceinline__ pair2 add2_rn(pair2 a, pair2 b) {
+    pair2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ pair2 add2_rz(pair2 a, pair2 b) {
+    pair2 d;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ pair2 fma2_rn(pair2 a, pair2 b, pair2 c) {
+    pair2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// Samples rows r, r + RS, ... of the rotated column `col` (row j of the frame
+// being jlo + row) into dst, zeros from row len on, dst rows < rows written.
+//
+// The y and x halves of a coordinate go through packed operations together:
+//   q = (Y (c, s) + (X (-s), X c)) + (o, o)     the reference's order
+//   u = q + 2^23 rounded down: 2^23 + floor(q); u - 2^23 the integer part, u
+//       plus (texel offset - 2^23) the texture coordinate
+//   f = q - floor(q) and 1 - f, exact and rounded once
+// instead of two conversions and eight more scalar operations per sample.
+// A packed multiply that feeds a packed add is fused with it on this part, whatever
+// its rounding qualifier says, so the product is an fma with an addend of -0
+// that the compiler cannot see through (a kernel argument): the product
+// rounded, as a multiply gives it.  The bilinear products stay scalar.
+//
+// kBounds = false when the texture's region sits at least two texels inside the
+// frame on every side (interior_source): a sample the reference's bounds
+// test rejects then has a stencil of border texels only (for q < 0 as well,
+// where u - 2^23 is q to a half), whose bilinear combination is +0, the value
+// the test would give.  Blocks of four rows all below len take no test at
+// all; the last one gathers only for rows below len.
+template <int RS, bool kBounds>
+__device__ __forceinline__ void sample_line(const BlockJob &J, float *dst, int col, int r, int jlo,
+                                            int len, int rows) {
+    const float o = (float)(J.n - 1) * 0.5f, nm1 = (float)(J.n - 1);
+    const float X = (float)col - o, big = 8388608.f;
+    const pair2 dir = pack2(J.c, J.s), base = pack2(__fmul_rn(X, -J.s), __fmul_rn(X, J.c));
+    const pair2 o2 = pack2(o, o), zero2 = pack2(J.neg_zero, J.neg_zero);
+    const pair2 big2 = pack2(big, big), nbig2 = pack2(-big, -big);
+    const pair2 tc2 = pack2(J.tu - big, J.tv - big);
+    const pair2 m1 = pack2(-1.f, -1.f), one2 = pack2(1.f, 1.f), step2 = pack2((float)RS, (float)RS);
+    const float Y0 = (float)(jlo + r) - o; // rows are integers below 2^24: exact throughout
+    pair2 Y = pack2(Y0, Y0);
+    // the coordinates of the next row and its gather
+    auto fetch = [&](float4 &g, pair2 &fr, bool &ok) {
+        const pair2 q = add2_rn(add2_rn(fma2_rn(Y, dir, zero2), base), o2);
+        const pair2 w = add2_rz(q, big2);
+        fr = fma2_rn(add2_rn(w, nbig2), m1, q);
+        const float2 tc = unpack2(add2_rn(w, tc2));
+        if (kBounds) {
+            const float2 p = unpack2(q);
+            ok = p.x >= 0.f && p.x < nm1 && p.y >= 0.f && p.y < nm1;
+        }
+        // texel (u, v) = image (row, col); w/z/x/y = s00, s10, s01, s11
+        g = tex2Dgather<float4>(J.tex, tc.x, tc.y, 0);
+        Y = add2_rn(Y, step2);
+    };
+    auto value = [&](const float4 &g, pair2 fr, bool ok) {
+        const float2 f = unpack2(fr), om = unpack2(fma2_rn(fr, m1, one2));
+        const float t0 = __fmul_rn(__fmul_rn(g.w, om.y), om.x);
+        const float t1 = __fmul_rn(__fmul_rn(g.x, f.y), om.x);
+        const float t2 = __fmul_rn(__fmul_rn(g.z, om.y), f.x);
+        const float t3 = __fmul_rn(__fmul_rn(g.y, f.y), f.x);
+        return ok ? __fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3) : 0.f;
+    };
+    constexpr int U = 4; // gathers in flight per thread
+    int i = 0;
+    for (; (i + U) * RS <= len; i += U) {
+        float4 g[U];
+        pair2 fr[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            ok[u] = true;
+            fetch(g[u], fr[u], ok[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            dst[r + RS * (i + u)] = value(g[u], fr[u], ok[u]);
+    }
+    int jr = r + RS * i;
+#pragma unroll 1
+    for (; i * RS < len; i++, jr += RS) { // at most U rows, one at a time
+        float4 g;
+        pair2 fr;
+        bool ok = true;
+        fetch(g, fr, ok);
+        if (jr < rows)
+            dst[jr] = value(g, fr, ok && jr < len);
+    }
+#pragma unroll 1
+    for (; jr < rows; jr += RS)
+        dst[jr] = 0.f;
+}
 
 // The fused body: support, sampling, T-functionals of one BlockJob.  Every
 // thread of the CTA (W >= L warps) calls it; it synchronises the CTA but
@@ -200,7 +349,6 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     const int n = J.n;
     const float c = J.c, s = J.s;
     const float o = (float)(n - 1) * 0.5f;
-    const float nm1 = (float)(n - 1);
     const int roff = J.roff, coff = J.coff;
     const int rr = max(J.rr, 0), rc = max(J.rc, 0);
 
@@ -229,51 +377,13 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     const int C = max((len + 31) >> 5, 1) | 1; // odd: conflict-free chunks
 
 
-    // 2. Sample the lines into shared memory (zeros past len, rows < 32 C).
+    // 2. Sample the lines into shared memory (zeros past len, rows < 32 C;
+    // lines past the frame are sampled too, no warp reads them).
     {
         constexpr int RS = 32 * W / L; // row streams per line
-        const int l = lane % L, r = (warp * 32 + lane) / L;
-        const int col = col0 + l;
-        const bool colok = col < n;
-        const float X = (float)col - o;
-        const float Xc = __fmul_rn(X, c), Xms = __fmul_rn(X, -s);
-        const float tu = J.tu, tv = J.tv;
-        float *dst = sm + l * stride;
-        const int rows = 32 * C, iters = (rows + RS - 1) / RS; // this thread: r + RS i
-        constexpr int U = 4;                                   // gathers in flight per thread
-        for (int i0 = 0; i0 < iters; i0 += U) {
-            float4 g[U];
-            float xf[U], yf[U];
-            bool ok[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int jr = r + RS * (i0 + u);
-                const float Y = (float)(jlo + jr) - o;
-                // (x c + y s) + o and (x (-s) + y c) + o, each operation rounded
-                const float qx = __fadd_rn(__fadd_rn(Xc, __fmul_rn(Y, s)), o);
-                const float qy = __fadd_rn(__fadd_rn(Xms, __fmul_rn(Y, c)), o);
-                ok[u] = colok && jr < len;
-                if (!kInterior) // see warp_sample: border texels answer the test
-                    ok[u] = ok[u] && qx >= 0.f && qx < nm1 && qy >= 0.f && qy < nm1;
-                const float xi = truncf(qx), yi = truncf(qy);
-                xf[u] = __fsub_rn(qx, xi);
-                yf[u] = __fsub_rn(qy, yi);
-                // texel (u, v) = image (row, col); w/z/x/y = s00, s10, s01, s11
-                g[u] = tex2Dgather<float4>(J.tex, yi + tu, xi + tv, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const float omx = __fsub_rn(1.f, xf[u]), omy = __fsub_rn(1.f, yf[u]);
-                const float t0 = __fmul_rn(__fmul_rn(g[u].w, omx), omy);
-                const float t1 = __fmul_rn(__fmul_rn(g[u].x, xf[u]), omy);
-                const float t2 = __fmul_rn(__fmul_rn(g[u].z, omx), yf[u]);
-                const float t3 = __fmul_rn(__fmul_rn(g[u].y, xf[u]), yf[u]);
-                const float v = __fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3);
-                const int jr = r + RS * (i0 + u);
-                if (jr < rows)
-                    dst[jr] = ok[u] ? v : 0.f;
-            }
-        }
+        const int l = lane % L;
+        sample_line<RS, !kInterior>(J, sm + l * stride, col0 + l, (warp * 32 + lane) / L, jlo, len,
+                                    32 * C);
     }
     __syncthreads();
 
@@ -328,28 +438,10 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     float r345[3] = {0.f, 0.f, 0.f};
     if (need & ((1u << 3) | (1u << 4) | (1u << 5))) {
         const bool w3 = need & (1u << 3), w4 = need & (1u << 4), w5 = need & (1u << 5);
-        const float2 *tab3 = J.tab, *tab4 = J.tab + n, *tab5 = J.tab + 2 * n;
         float re3 = 0.f, im3 = 0.f, re4 = 0.f, im4 = 0.f, re5 = 0.f, im5 = 0.f;
         const int lo = max(1, jlo - m2), hi = min(n - m2, jhi - m2);
-#pragma unroll 4
-        for (int q = lo + lane; q < hi; q += 32) {
-            const float v = x[m2 + q - jlo];
-            if (w3) {
-                const float2 w = __ldg(tab3 + q);
-                re3 = fmaf(w.x, v, re3);
-                im3 = fmaf(w.y, v, im3);
-            }
-            if (w4) {
-                const float2 w = __ldg(tab4 + q);
-                re4 = fmaf(w.x, v, re4);
-                im4 = fmaf(w.y, v, im4);
-            }
-            if (w5) {
-                const float2 w = __ldg(tab5 + q);
-                re5 = fmaf(w.x, v, re5);
-                im5 = fmaf(w.y, v, im5);
-            }
-        }
+        tail345<32>(J.tab, n, x + (m2 - jlo), lo + lane, hi, w3, w4, w5, re3, im3, re4, im4, re5,
+                    im5);
         // hypot of the two float integrals (CUDA's hypotf: no FP64, whose
         // narrow pipe every lane of every line would otherwise queue on)
         if (w3)
@@ -394,8 +486,15 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     } // col < n
 }
 
+// CTAs per SM the registers should allow: as many as the line buffers do at
+// their shortest (64 registers a thread; 80 with the selections, whose
+// histograms leave room for three CTAs of 8 lines).
+constexpr int sino_min_ctas(int L, int W, bool sel) {
+    return W > L ? 2 : (sel ? 24 : 32) / L;
+}
+
 template <int L, bool kSel, bool kInterior, int W = L>
-__global__ void __launch_bounds__(32 * W, W > L ? 2 : 1)
+__global__ void __launch_bounds__(32 * W, sino_min_ctas(L, W, kSel))
     sino_kernel(const SinoArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_range[2];
@@ -429,6 +528,7 @@ __global__ void __launch_bounds__(32 * W, W > L ? 2 : 1)
     J.coff = s_region[1];
     J.rr = s_region[2];
     J.rc = s_region[3];
+    J.neg_zero = a.neg_zero;
     J.tab = a.tab;
     J.out = a.out;
     J.medians = a.medians;
@@ -444,7 +544,7 @@ __global__ void __launch_bounds__(32 * W, W > L ? 2 : 1)
 // counts: each CTA claims work items (image, angle, line block) from a
 // counter until all are taken; items are numbered largest image first.
 template <int L, bool kSel, bool kInterior>
-__global__ void __launch_bounds__(32 * L)
+__global__ void __launch_bounds__(32 * L, sino_min_ctas(L, L, kSel))
     sino_batch_kernel(const BatchSinoArgs b) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_range[2];
@@ -481,6 +581,7 @@ __global__ void __launch_bounds__(32 * L)
         J.coff = im.col_off;
         J.rr = im.rows;
         J.rc = im.cols;
+        J.neg_zero = b.neg_zero;
         J.tab = b.tab + im.tab_off;
         J.out = b.sino + im.sino_off;
         J.medians = nullptr;
@@ -652,58 +753,18 @@ __host__ __device__ constexpr int warp_line_stride(int n, int lpw) {
            (32 / lpw) % 32;
 }
 
-// Sampling of the warp-autonomous path: lane (s, sub) takes rows sub + SW i
-// of line s into x.  kBounds = false when the texture's region sits at least
-// two texels inside the frame on every side (interior_source): a sample the
-// reference's bounds test rejects then has a stencil of border texels only,
-// whose bilinear combination is +0, the value the test would give.
-template <int SW, bool kBounds>
-__device__ __forceinline__ void warp_sample(const BlockJob &J, float *x, int col, bool colok,
-                                            int jlo, int len, int C, int sub) {
-    const int n = J.n;
-    const float c = J.c, sn = J.s;
-    const float o = (float)(n - 1) * 0.5f, nm1 = (float)(n - 1);
-    const float X = (float)col - o;
-    const float Xc = __fmul_rn(X, c), Xms = __fmul_rn(X, -sn);
-    const float tu = J.tu, tv = J.tv;
-    constexpr int U = 4;
-    float Y0 = (float)(jlo + sub) - o; // exact: integers below 2^24
-    for (int i0 = 0; i0 < C; i0 += U) {
-        float4 g[U];
-        float xf[U], yf[U];
-        bool ok[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int jr = sub + SW * (i0 + u);
-            const float Y = Y0 + (float)(SW * u);
-            const float qx = __fadd_rn(__fadd_rn(Xc, __fmul_rn(Y, sn)), o);
-            const float qy = __fadd_rn(__fadd_rn(Xms, __fmul_rn(Y, c)), o);
-            ok[u] = colok && jr < len;
-            if (kBounds)
-                ok[u] = ok[u] && qx >= 0.f && qx < nm1 && qy >= 0.f && qy < nm1;
-            const float xi = truncf(qx), yi = truncf(qy);
-            xf[u] = __fsub_rn(qx, xi);
-            yf[u] = __fsub_rn(qy, yi);
-            g[u] = tex2Dgather<float4>(J.tex, yi + tu, xi + tv, 0);
-        }
-        Y0 += (float)(SW * U);
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const float omx = __fsub_rn(1.f, xf[u]), omy = __fsub_rn(1.f, yf[u]);
-            const float t0 = __fmul_rn(__fmul_rn(g[u].w, omx), omy);
-            const float t1 = __fmul_rn(__fmul_rn(g[u].x, xf[u]), omy);
-            const float t2 = __fmul_rn(__fmul_rn(g[u].z, omx), yf[u]);
-            const float t3 = __fmul_rn(__fmul_rn(g[u].y, xf[u]), yf[u]);
-            const float v = __fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3);
-            if (i0 + u < C)
-                x[sub + SW * (i0 + u)] = ok[u] ? v : 0.f;
-        }
-    }
-}
+// Where a warp's lines go and the kernels of their length: read after the
+// sampling, which needs the registers (late() in warp_lines).
+struct LineOut {
+    const float2 *tab;
+    float *out;
+    int32_t *medians;
+    size_t plane;
+};
 
-template <int LPW, bool kInterior>
+template <int LPW, bool kInterior, class Late>
 __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_t,
-                           unsigned need, int stride, float *xw) {
+                           unsigned need, int stride, float *xw, Late late) {
     constexpr int SW = 32 / LPW;
     const int lane = threadIdx.x & 31, s = lane / SW, sub = lane % SW;
     const int n = J.n, angle = J.angle;
@@ -730,8 +791,9 @@ __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_
     float *x = xw + s * stride;
 
     // 2. sampling
-    warp_sample<SW, !kInterior>(J, x, col, colok, jlo, len, C, sub);
+    sample_line<SW, !kInterior>(J, x, col, sub, jlo, len, SW * C);
     __syncwarp();
+    const LineOut O = late();
 
     // 3. T0-T5 of each segment's line
     const bool need_m1 = need & ((1u << 1) | (1u << 2));
@@ -781,26 +843,9 @@ __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_
     float re3 = 0.f, im3 = 0.f, re4 = 0.f, im4 = 0.f, re5 = 0.f, im5 = 0.f;
     if (need_m2) {
         const bool w3 = need & (1u << 3), w4 = need & (1u << 4), w5 = need & (1u << 5);
-        const float2 *tab3 = J.tab, *tab4 = J.tab + n, *tab5 = J.tab + 2 * n;
         const int qlo = max(1, jlo - m2), qhi = min(n - m2, jhi - m2);
-        for (int q = qlo + sub; q < qhi; q += SW) {
-            const float v = x[m2 + q - jlo];
-            if (w3) {
-                const float2 w = __ldg(tab3 + q);
-                re3 = fmaf(w.x, v, re3);
-                im3 = fmaf(w.y, v, im3);
-            }
-            if (w4) {
-                const float2 w = __ldg(tab4 + q);
-                re4 = fmaf(w.x, v, re4);
-                im4 = fmaf(w.y, v, im4);
-            }
-            if (w5) {
-                const float2 w = __ldg(tab5 + q);
-                re5 = fmaf(w.x, v, re5);
-                im5 = fmaf(w.y, v, im5);
-            }
-        }
+        tail345<SW>(O.tab, n, x + (m2 - jlo), qlo + sub, qhi, w3, w4, w5, re3, im3, re4, im4, re5,
+                    im5);
     }
 
     // 4. the eight sums of a segment reduced transposed: after the halving
@@ -814,16 +859,16 @@ __device__ void warp_lines(const BlockJob &J, unsigned long long tf_code, int n_
     const float other = __shfl_xor_sync(TT_FULL_MASK, v8, unit);
     const float res = k8 >= 2 ? hypotf(k8 & 1 ? other : v8, k8 & 1 ? v8 : other) : v8;
     // n_t <= kWarpMaxOutputs <= SW (the hosts' choice of this path)
-    const size_t plane = J.plane;
+    const size_t plane = O.plane;
     const size_t at = (size_t)angle * n + col;
     const int t = sub < n_t ? sub : 0;
     const int f = (int)((tf_code >> (3 * t)) & 7ull);
     const int kf = f == 1 ? 0 : f == 2 ? 1 : f == 3 ? 2 : f == 4 ? 4 : 6;
     const float got = __shfl_sync(TT_FULL_MASK, res, s * SW + kf * unit);
     if (colok && sub < n_t) {
-        J.out[t * plane + at] = f == 0 ? S : got;
-        if (J.medians)
-            J.medians[t * plane + at] = f == 0 ? -1 : f <= 2 ? m1 : m2;
+        O.out[t * plane + at] = f == 0 ? S : got;
+        if (O.medians)
+            O.medians[t * plane + at] = f == 0 ? -1 : f <= 2 ? m1 : m2;
     }
 }
 
@@ -855,15 +900,15 @@ __global__ void __launch_bounds__(32 * W, 32 / W) sino_warp_kernel(const SinoArg
         J.rr = a.src_rows;
         J.rc = a.src_cols;
     }
-    J.tab = a.tab;
-    J.out = a.out;
-    J.medians = a.medians;
-    J.plane = (size_t)a.n_angles * a.n;
+    J.neg_zero = a.neg_zero;
     unsigned long long code = 0;
     for (int t = 0; t < a.n_t; t++)
         code |= (unsigned long long)(a.tf[t] & 7) << (3 * t);
     warp_lines<LPW, kInterior>(J, code, a.n_t, a.need, a.stride,
-                               smw + (size_t)warp * LPW * a.stride);
+                               smw + (size_t)warp * LPW * a.stride, [&]() {
+                                   return LineOut{a.tab, a.out, a.medians,
+                                                  (size_t)a.n_angles * a.n};
+                               });
 }
 
 // Batch: every warp claims (image, angle, LPW-line block) items from the
@@ -908,11 +953,12 @@ __global__ void __launch_bounds__(32 * W, 32 / W) sino_batch_warp_kernel(const B
         J.coff = im.col_off;
         J.rr = im.rows;
         J.rc = im.cols;
-        J.tab = b.tab + im.tab_off;
-        J.out = b.sino + im.sino_off;
-        J.medians = nullptr;
-        J.plane = (size_t)im.n_angles * im.n;
-        warp_lines<LPW, kInterior>(J, b.tf_code, b.n_t, b.need, b.stride, xw);
+        J.neg_zero = b.neg_zero;
+        warp_lines<LPW, kInterior>(J, b.tf_code, b.n_t, b.need, b.stride, xw, [&]() {
+            const BatchImage &d = b.img[lo];
+            return LineOut{b.tab + d.tab_off, b.sino + d.sino_off, nullptr,
+                           (size_t)d.n_angles * d.n};
+        });
         __syncwarp(); // the line rows are rewritten by the next item
     }
 }
