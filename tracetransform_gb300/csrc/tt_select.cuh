@@ -31,13 +31,33 @@
 namespace tt {
 
 constexpr int kSelBins = 256;
-constexpr int kSelList = 192; // collected entries (in the histogram's place)
+constexpr int kSelList = 188; // collected entries (in the histogram's place)
 
+struct SelPick {
+    unsigned bin, below, total;
+};
 struct __align__(16) SelScratch {
     union {
         unsigned hist[kSelBins];
         uint2 list[kSelList]; // key bits, then the sample's bits or its weight
     };
+    // several warps on one line: its pick, the weight at the largest sample,
+    // the entries collected
+    SelPick pick;
+    unsigned wtop;
+    int count;
+};
+static_assert(sizeof(SelScratch) == 1536, "the lines per CTA and line lengths it allows");
+
+// The TW warps of a line: this warp's place among them and their barrier.
+template <int TW> struct SelTeam {
+    int role, bar;
+    __device__ __forceinline__ void sync() const {
+        if (TW == 1)
+            __syncwarp();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * TW) : "memory");
+    }
 };
 
 // Fixed-point weight of a sample v: sqrt(v) (T6, T7) or v itself (P2).
@@ -81,9 +101,6 @@ __device__ __forceinline__ void sel_clear(SelScratch *sc, int lane) {
 // it) >= total.  On entry `below` is the weight of all keys under the
 // histogram's range, on return that of all keys under the bin.  kTotal: the
 // histogram holds every weight, its sum is the total.
-struct SelPick {
-    unsigned bin, below, total;
-};
 template <bool kTotal>
 __device__ __forceinline__ SelPick sel_pick(const SelScratch *sc, unsigned below, unsigned total,
                                             int lane) {
@@ -132,10 +149,19 @@ struct SelTest {
 };
 
 // Append (key, sample) of the lanes with `in` set to the list (counted past
-// its end, never written there).
+// its end, never written there); kTeam: several warps append to it.
+template <bool kTeam = false>
 __device__ __forceinline__ void sel_append(SelScratch *sc, int &count, bool in, float k, float v,
                                            int lane) {
     const unsigned m = __ballot_sync(TT_FULL_MASK, in);
+    if (kTeam) {
+        if (!m)
+            return;
+        int at = 0;
+        if (lane == 0)
+            at = atomicAdd(&sc->count, __popc(m));
+        count = __shfl_sync(TT_FULL_MASK, at, 0);
+    }
     const int pos = count + __popc(m & ((1u << lane) - 1u));
     if (in && pos < kSelList)
         sc->list[pos] = make_uint2(__float_as_uint(k), __float_as_uint(v));
@@ -218,6 +244,23 @@ __device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, 
     return klo;
 }
 
+// Clears a line's two histograms; before the team's next sync, which comes
+// before select_t67.
+template <int TW>
+__device__ __forceinline__ void sel_begin(SelScratch *s6, SelScratch *s7, SelTeam<TW> team,
+                                          int lane) {
+    if (TW == 1 || team.role == TW - 1)
+        sel_clear(s7, lane);
+    if (TW == 1 || team.role == TW - 2)
+        sel_clear(s6, lane);
+    if (TW > 1 && team.role == TW - 1 && lane == 0) {
+        s7->wtop = 0u;
+        s7->count = s6->count = 0;
+    }
+    if (TW == 1)
+        __syncwarp();
+}
+
 // T6 and T7 of one line (c++/src/functionals.cpp:226-276).  T6: keys
 // r1 * x[m2 + r1], r1 in [0, N - m2); T7: keys x[m1 ..]; both weighted by
 // sqrt(x).  Elements are the line's stored rows at x[row - jlo]; every other
@@ -227,11 +270,13 @@ __device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, 
 // chunked sweep: far-apart elements in flight, so fewer atomic collisions).
 // xmax and qtot (the line's largest sample and sum of square roots) bound
 // every key and weight total, so no separate range pass is needed; odd: some
-// sample is none sqrt_pos takes.
-inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int m2, bool want6,
-                                  bool want7, float xmax, float qtot, bool odd,
-                                  SelScratch *s6, SelScratch *s7, int lane, float *r6,
-                                  float *r7) {
+// sample is none sqrt_pos takes.  The line's TW warps share both passes; T7's
+// answer is the first one's, T6's the second one's (TW = 1: both its own).
+template <int TW>
+__device__ __forceinline__ void select_t67(const float *x, int jlo, int jhi, int m1, int m2,
+                                           bool want6, bool want7, float xmax, float qtot,
+                                           bool odd, SelScratch *s6, SelScratch *s7,
+                                           SelTeam<TW> team, int lane, float *r6, float *r7) {
     *r6 = 0.f;
     *r7 = 0.f;
     const int b7 = max(m1, jlo), b6 = max(m2, jlo);
@@ -239,7 +284,7 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
     const int cnt = jhi - b;
     if (cnt <= 0 || !(xmax > 0.f) || !(qtot > 0.f))
         return;
-    const int per = ((cnt + 31) >> 5) | 1; // odd: conflict-free chunks
+    const int per = ((cnt + 32 * TW - 1) / (32 * TW)) | 1; // odd: conflict-free chunks
     const SqrtWeight wfn{sel_scale(qtot), odd};
     const float k6max = __fmul_rn((float)max(jhi - 1 - m2, 0), xmax);
     want6 = want6 && k6max > 0.f; // otherwise every T6 key is 0
@@ -247,13 +292,10 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
     // element e of [0, cnt) is row b + e; this lane's are e0 .. e0 + mine - 1,
     // of which T7 takes those from i = f7 on and T6 those from f6
     const float *xb = x + (b - jlo);
-    const int e0 = lane * per, mine = min(max(cnt - e0, 0), per);
+    const int e0 = (team.role * 32 + lane) * per, mine = min(max(cnt - e0, 0), per);
     const int f7 = want7 ? b7 - b - e0 : per, f6 = want6 ? b6 - b - e0 : per;
     const float r0 = (float)(b + e0 - m2); // T6's factor of the lane's first element
 
-    sel_clear(s6, lane);
-    sel_clear(s7, lane);
-    __syncwarp();
     unsigned l7max = 0;
     float rf = r0; // exact: integers below 2^24
     // a warp-uniform trip count (per), lanes past their chunk predicated off
@@ -274,24 +316,37 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
                 atomicAdd(s6->hist + sel_bin(__fmul_rn(rf + (float)u, v), 0.f, bs6), wq);
         }
     }
-    __syncwarp();
+    unsigned wtop = __reduce_add_sync(TT_FULL_MASK, l7max);
+    if (TW > 1 && lane == 0 && wtop)
+        atomicAdd(&s7->wtop, wtop);
+    team.sync();
     SelPick p7{0u, 0u, 0u}, p6{0u, 0u, 0u};
-    if (want7) {
+    const int own6 = TW > 1 ? 1 : 0; // the warp that finishes T6
+    if (want7 && team.role == 0)
         p7 = sel_pick<true>(s7, 0u, 0u, lane);
-        // Saturated lines (samples clipped at the image's maximum) put the
-        // crossing on the largest key: when the keys below the maximum weigh
-        // less than half the total, 2 W(< xmax) < W, the answer is xmax.
-        const unsigned wmax = __reduce_add_sync(TT_FULL_MASK, l7max);
-        if (wmax > 0 && 2u * (p7.total - wmax) < p7.total) {
-            *r7 = xmax;
-            want7 = false;
-        }
-    }
-    if (want6)
+    if (want6 && team.role == own6)
         p6 = sel_pick<true>(s6, 0u, 0u, lane);
+    if (TW > 1) {
+        if (lane == 0 && team.role == 0)
+            s7->pick = p7;
+        if (lane == 0 && team.role == own6)
+            s6->pick = p6;
+    }
+    team.sync(); // both histograms are read: the lists take their place
+    if (TW > 1) {
+        p7 = s7->pick;
+        p6 = s6->pick;
+        wtop = s7->wtop;
+    }
+    // Saturated lines (samples clipped at the image's maximum) put the
+    // crossing on the largest key: when the keys below the maximum weigh
+    // less than half the total, 2 W(< xmax) < W, the answer is xmax.
+    if (want7 && wtop > 0 && 2u * (p7.total - wtop) < p7.total) {
+        *r7 = xmax;
+        want7 = false;
+    }
     if (!want6 && !want7)
         return;
-    __syncwarp(); // both histograms are read: the lists take their place
     const SelTest in7(0.f, bs7, p7.bin), in6(0.f, bs6, p6.bin);
     int c6 = 0, c7 = 0;
     rf = r0;
@@ -307,13 +362,17 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
             const bool a7 = want7 && i >= f7 && i < mine && in7(v);
             const bool a6 = want6 && i >= f6 && i < mine && in6(k6);
             if (__any_sync(TT_FULL_MASK, a7 || a6)) {
-                sel_append(s7, c7, a7, v, v, lane);
-                sel_append(s6, c6, a6, k6, v, lane);
+                sel_append<(TW > 1)>(s7, c7, a7, v, v, lane);
+                sel_append<(TW > 1)>(s6, c6, a6, k6, v, lane);
             }
         }
     }
-    __syncwarp();
-    if (want7) {
+    team.sync();
+    if (TW > 1) {
+        c7 = s7->count;
+        c6 = s6->count;
+    }
+    if (want7 && team.role == 0) {
         if (c7 <= kSelList) {
             *r7 = sel_answer(s7, c7, p7.below, p7.total, wfn, lane);
         } else {
@@ -322,7 +381,7 @@ inline __device__ void select_t67(const float *x, int jlo, int jhi, int m1, int 
                              lane);
         }
     }
-    if (want6) {
+    if (want6 && team.role == own6) {
         if (c6 <= kSelList) {
             *r6 = sel_answer(s6, c6, p6.below, p6.total, wfn, lane);
         } else {

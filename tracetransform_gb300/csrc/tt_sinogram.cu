@@ -269,8 +269,14 @@ __device__ __forceinline__ pair2 fma2_rn(pair2 a, pair2 b, pair2 c) {
 // frame on every side (interior_source): a sample the reference's bounds
 // test rejects then has a stencil of border texels only (for q < 0 as well,
 // where u - 2^23 is q to a half), whose bilinear combination is +0, the value
-// the test would give.  Blocks of four rows all below len take no test at
-// all; the last one gathers only for rows below len.
+// the test would give.  Four rows at a time while all are below len, then
+// one at a time: no gather is spent on rows past len (in a rolled loop: the
+// unrolled form spilled in the persistent kernels).
+//
+// Bound: the texture unit's write-back, 16 bytes per sample or 16 cycles per
+// warp and gather (88 % busy with T0 alone at 1024^2).  T0 of 389 x 640 x 360
+// angles: 178 us, of 1024^2 x 360: 714 us (194 and 782 with scalar coordinates,
+// conversions and gathers up to the next four rows).
 template <int RS, bool kBounds>
 __device__ __forceinline__ void sample_line(const BlockJob &J, float *dst, int col, int r, int jlo,
                                             int len, int rows) {
@@ -335,14 +341,53 @@ __device__ __forceinline__ void sample_line(const BlockJob &J, float *dst, int c
         dst[jr] = 0.f;
 }
 
+// Eight sums over a segment of SW >= 8 lanes, transposed: three halving
+// exchanges (each lane keeps the half of the values its offset bit selects
+// and adds its partner's copy of it), then plain butterflies over the rest;
+// lane sub ends with sum k = (sub / (SW / 8)) % 8 of (a0, ..., a7).
+template <int SW>
+__device__ __forceinline__ float seg_sum8(float a0, float a1, float a2, float a3, float a4,
+                                          float a5, float a6, float a7, int sub) {
+    static_assert(SW >= 8, "eight sums need eight lanes");
+    constexpr int d1 = SW / 2, d2 = SW / 4, d3 = SW / 8;
+    bool hi = sub & d1; // keep a4..a7
+    float k0 = hi ? a4 : a0, k1 = hi ? a5 : a1, k2 = hi ? a6 : a2, k3 = hi ? a7 : a3;
+    const float s0 = hi ? a0 : a4, s1 = hi ? a1 : a5, s2 = hi ? a2 : a6, s3 = hi ? a3 : a7;
+    k0 += __shfl_xor_sync(TT_FULL_MASK, s0, d1);
+    k1 += __shfl_xor_sync(TT_FULL_MASK, s1, d1);
+    k2 += __shfl_xor_sync(TT_FULL_MASK, s2, d1);
+    k3 += __shfl_xor_sync(TT_FULL_MASK, s3, d1);
+    hi = sub & d2; // keep k2, k3
+    float m0 = hi ? k2 : k0, m1 = hi ? k3 : k1;
+    const float t0 = hi ? k0 : k2, t1 = hi ? k1 : k3;
+    m0 += __shfl_xor_sync(TT_FULL_MASK, t0, d2);
+    m1 += __shfl_xor_sync(TT_FULL_MASK, t1, d2);
+    hi = sub & d3; // keep m1
+    float r = hi ? m1 : m0;
+    r += __shfl_xor_sync(TT_FULL_MASK, hi ? m0 : m1, d3);
+#pragma unroll
+    for (int d = d3 / 2; d > 0; d >>= 1)
+        r += __shfl_xor_sync(TT_FULL_MASK, r, d);
+    return r;
+}
+
+// What the warps of a line's team tell one another (TW > 1: 80 bytes a line,
+// small enough that the longest line the shared memory takes still fits).
+template <int TW> struct LineShare {
+    float S, Q, top;
+    short m1, m2;     // m1 complemented: the line holds odd samples
+    float part[2][8]; // the second and third warp's tail sums
+};
+template <> struct LineShare<1> {};
+
 // The fused body: support, sampling, T-functionals of one BlockJob.  Every
-// thread of the CTA (W >= L warps) calls it; it synchronises the CTA but
-// never returns early.  All W warps sample; warps 0..L-1 then take one line
+// thread of the CTA (W >= L warps) calls it; it synchronises the CTA (before
+// the functionals only).  All W warps sample; W / L warps then take a line
 // each.  tf_code holds the T-functional id of output t in bits [3t, 3t + 3).
 template <int L, bool kSel, bool kInterior, int W = L>
 __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long tf_code,
                                            int n_t, unsigned need, int stride, float *sm,
-                                           int *s_range) {
+                                           int *s_range, LineShare<W / L> *share) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int angle = J.angle;
     const int col0 = J.col0;
@@ -387,42 +432,82 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
     }
     __syncthreads();
 
-    // 3. One warp per line: T-functionals.
-    const int col = col0 + warp;
-    if (warp < L && col < n) {
-    float *x = sm + warp * stride;
+    // 3. T-functionals: TW warps per line.  The chunk sums and medians are
+    // sequential by their definition, so one warp takes the plain ones and
+    // another the square roots'; the tails, the histograms and the collecting
+    // are shared by rows.  Long lines (W > L) run 4 lines per CTA and 2 CTAs
+    // per SM, so with one warp per line 8 warps per SM had all the
+    // functionals to do: 4096^2 x 720 angles, T0-T7: 65.6 ms, from 84.7.
+    constexpr int TW = W / L;
+    static_assert(TW == 1 || TW == 4, "the roles below");
+    // a team's warps sit on the four schedulers, its roles rotated by line
+    const int line = warp / TW, role = (warp + line) % TW;
+    const int col = col0 + line;
+    const bool alone = TW > 1 && (need & ~1u) == 0; // T0: the first warp's own
+    if (col >= n || (alone && role > 0))
+        return; // the whole team, or all it does not need
+    const float *x = sm + line * stride;
+    const SelTeam<TW> team{role, 1 + line};
+    SelScratch *scr = reinterpret_cast<SelScratch *>(sm + L * stride) + 2 * line; // kSel only
     const bool need_m1 = need & ((1u << 1) | (1u << 2) | (1u << 7));
     const bool need_m2 = need & ((1u << 3) | (1u << 4) | (1u << 5) | (1u << 6));
     const bool need_sq = need_m2 || (need & (1u << 7)); // sum of sqrt(x) wanted
-    const int base = lane * C;
-
-    const ChunkSums cs = need_sq ? chunk_sums<true>(x + base, C) : chunk_sums<false>(x + base, C);
-    const float inc = warp_incl_scan(cs.tot, lane);
-    const float S = __shfl_sync(TT_FULL_MASK, inc, 31);
-    float exc = __shfl_up_sync(TT_FULL_MASK, inc, 1);
-    float Q = 0.f, incq = 0.f, excq = 0.f;
-    if (need_sq) {
-        incq = warp_incl_scan(cs.totq, lane);
-        Q = __shfl_sync(TT_FULL_MASK, incq, 31);
-        excq = __shfl_up_sync(TT_FULL_MASK, incq, 1);
-    }
-    if (lane == 0) {
-        exc = 0.f;
-        excq = 0.f;
-    }
-
+    const bool plain = TW == 1 || role == 0, roots = need_sq && (TW == 1 || role == 1);
+    if (kSel)
+        sel_begin(scr, scr + 1, team, lane);
+    float S = 0.f, Q = 0.f, top = 0.f;
     int m1 = 0, m2 = 0;
-    if (need_m1) {
-        const int f = cs.neg ? find_crossing_walk(x, C, exc, S, lane)
-                              : find_crossing<false>(x, C, inc, exc, S, false, lane);
-        m1 = resolve_median(f, S, jlo, jhi, len, n);
+    bool odd = false;
+    if (plain || roots) {
+        const float *xc = x + lane * C;
+        const ChunkSums cs = roots ? chunk_sums<true>(xc, C) : chunk_sums<false>(xc, C);
+        odd = cs.odd;
+        if (plain) {
+            const float inc = warp_incl_scan(cs.tot, lane);
+            S = __shfl_sync(TT_FULL_MASK, inc, 31);
+            float exc = __shfl_up_sync(TT_FULL_MASK, inc, 1);
+            exc = lane ? exc : 0.f;
+            top = __int_as_float(warp_max(__float_as_int(cs.top)));
+            if (need_m1) {
+                const int f = cs.neg ? find_crossing_walk(x, C, exc, S, lane)
+                                     : find_crossing<false>(x, C, inc, exc, S, false, lane);
+                m1 = resolve_median(f, S, jlo, jhi, len, n);
+            }
+        }
+        if (roots) {
+            const float inc = warp_incl_scan(cs.totq, lane);
+            Q = __shfl_sync(TT_FULL_MASK, inc, 31);
+            float exc = __shfl_up_sync(TT_FULL_MASK, inc, 1);
+            exc = lane ? exc : 0.f;
+            if (need_m2)
+                m2 = resolve_median(find_crossing<true>(x, C, inc, exc, Q, odd, lane), Q, jlo,
+                                    jhi, len, n);
+        }
     }
-    if (need_m2)
-        m2 = resolve_median(find_crossing<true>(x, C, incq, excq, Q, cs.odd, lane), Q, jlo, jhi, len, n);
+    LineShare<TW> &sh = share[line];
+    if constexpr (TW > 1) if (!alone) {
+        if (lane == 0 && role == 0) {
+            sh.S = S;
+            sh.top = top;
+            sh.m1 = (short)(odd ? ~m1 : m1); // below 2^15: n is bounded by shared memory
+        }
+        if (lane == 0 && role == 1) {
+            sh.Q = Q;
+            sh.m2 = (short)m2;
+        }
+        team.sync();
+        S = sh.S;
+        Q = sh.Q;
+        top = sh.top;
+        m2 = sh.m2;
+        odd = sh.m1 < 0;
+        m1 = odd ? ~(int)sh.m1 : sh.m1;
+    }
 
-    float r1v = 0.f, r2v = 0.f;
-    if (need & ((1u << 1) | (1u << 2))) {
-        float t1 = 0.f, t2 = 0.f;
+    float t1 = 0.f, t2 = 0.f, re3 = 0.f, im3 = 0.f, re4 = 0.f, im4 = 0.f, re5 = 0.f, im5 = 0.f;
+    // a team's third warp takes T1 and T2 (in one warp's order, as gradients of P1
+    // hang on their last bits), the other three T3-T5
+    if (need & ((1u << 1) | (1u << 2)) && (TW == 1 || role == 2)) {
 #pragma unroll 4
         for (int j = max(m1, jlo) + lane; j < jhi; j += 32) {
             const float v = x[j - jlo];
@@ -431,59 +516,62 @@ __device__ __forceinline__ void sino_block(const BlockJob &J, unsigned long long
             t1 += vr;
             t2 = fmaf(vr, r, t2);
         }
-        r1v = warp_sum(t1);
-        r2v = warp_sum(t2);
     }
-
-    float r345[3] = {0.f, 0.f, 0.f};
-    if (need & ((1u << 3) | (1u << 4) | (1u << 5))) {
-        const bool w3 = need & (1u << 3), w4 = need & (1u << 4), w5 = need & (1u << 5);
-        float re3 = 0.f, im3 = 0.f, re4 = 0.f, im4 = 0.f, re5 = 0.f, im5 = 0.f;
-        const int lo = max(1, jlo - m2), hi = min(n - m2, jhi - m2);
-        tail345<32>(J.tab, n, x + (m2 - jlo), lo + lane, hi, w3, w4, w5, re3, im3, re4, im4, re5,
-                    im5);
-        // hypot of the two float integrals (CUDA's hypotf: no FP64, whose
-        // narrow pipe every lane of every line would otherwise queue on)
-        if (w3)
-            r345[0] = hypotf(warp_sum(re3), warp_sum(im3));
-        if (w4)
-            r345[1] = hypotf(warp_sum(re4), warp_sum(im4));
-        if (w5)
-            r345[2] = hypotf(warp_sum(re5), warp_sum(im5));
+    if (need & ((1u << 3) | (1u << 4) | (1u << 5)) && (TW == 1 || role != 2))
+        tail345<TW == 1 ? 32 : 32 * (TW - 1)>(
+            J.tab, n, x + (m2 - jlo), max(1, jlo - m2) + 32 * min(role, 2) + lane,
+            min(n - m2, jhi - m2), need & (1u << 3), need & (1u << 4), need & (1u << 5), re3, im3,
+            re4, im4, re5, im5);
+    // lane 4 k of the warp holds sum k of (t1, t2, re3, im3, re4, im4, re5, im5)
+    const bool tails = need & 0x3eu, moduli = need & 0x38u;
+    float v8 = 0.f;
+    float *part3 = sm + line * stride + stride - 8; // TW > 1: the line's spare floats
+    if (tails) {
+        if (moduli) {
+            v8 = seg_sum8<32>(t1, t2, re3, im3, re4, im4, re5, im5, lane);
+        } else { // T1 and T2 alone: the same sums
+            t1 = warp_sum(t1);
+            t2 = warp_sum(t2);
+            v8 = lane < 4 ? t1 : t2;
+        }
+        if constexpr (TW > 1)
+            if (role > 0 && (lane & 3) == 0)
+                (role < 3 ? sh.part[role - 1] : part3)[lane >> 2] = v8;
     }
 
     float r6v = 0.f, r7v = 0.f;
-    if (kSel) {
-        SelScratch *scr = reinterpret_cast<SelScratch *>(sm + L * stride) + 2 * warp;
-        const float xmax = __int_as_float(warp_max(__float_as_int(cs.top)));
+    if (kSel)
         // T6: keys r1 * x[m2 + r1], r1 in [0, N - m2); T7: keys x[m1 ..]
-        select_t67(x, jlo, jhi, m1, m2, need & (1u << 6), need & (1u << 7), xmax, Q, cs.odd, scr,
-                   scr + 1, lane, &r6v, &r7v);
-    }
-
-    if (lane == 0) {
-        const size_t plane = J.plane;
-        const size_t at = (size_t)angle * n + col;
-        for (int t = 0; t < n_t; t++) {
-            const int f = (int)((tf_code >> (3 * t)) & 7ull);
-            float v;
-            int med;
-            switch (f) {
-            case 0: v = S; med = -1; break;
-            case 1: v = r1v; med = m1; break;
-            case 2: v = r2v; med = m1; break;
-            case 3: v = r345[0]; med = m2; break;
-            case 4: v = r345[1]; med = m2; break;
-            case 5: v = r345[2]; med = m2; break;
-            case 6: v = r6v; med = m2; break;
-            default: v = r7v; med = m1; break;
-            }
-            J.out[t * plane + at] = v;
-            if (J.medians)
-                J.medians[t * plane + at] = med;
+        select_t67(x, jlo, jhi, m1, m2, need & (1u << 6), need & (1u << 7), top, Q, odd, scr,
+                   scr + 1, team, lane, &r6v, &r7v);
+    float res = 0.f;
+    if (tails) {
+        if constexpr (TW > 1) {
+            team.sync(); // the parts are in place
+            if (role == 0)
+                v8 += (sh.part[0][lane >> 2] + sh.part[1][lane >> 2]) + part3[lane >> 2];
+        }
+        res = v8;
+        if (moduli) { // |re + i im| on lanes 8 .. 31 (CUDA's hypotf: no FP64)
+            const int k8 = lane >> 2;
+            const float other = __shfl_xor_sync(TT_FULL_MASK, v8, 4);
+            res = k8 >= 2 ? hypotf(k8 & 1 ? other : v8, k8 & 1 ? v8 : other) : v8;
         }
     }
-    } // col < n
+    // lane t writes output t
+    const int t = lane < n_t ? lane : 0;
+    const int f = (int)((tf_code >> (3 * t)) & 7ull);
+    const float got = __shfl_sync(TT_FULL_MASK, res, f == 1 ? 0 : f == 2 ? 4 : f == 3 ? 8
+                                                                   : f == 4   ? 16
+                                                                              : 24);
+    const float v = f == 0 ? S : f == 6 ? r6v : f == 7 ? r7v : got;
+    // T6's answer is held by the team's second warp, everything else by its first
+    if (lane < n_t && role == (TW > 1 && f == 6 ? 1 : 0)) {
+        const size_t plane = J.plane, at = (size_t)angle * n + col;
+        J.out[t * plane + at] = v;
+        if (J.medians)
+            J.medians[t * plane + at] = f == 0 ? -1 : f <= 2 || f == 7 ? m1 : m2;
+    }
 }
 
 // CTAs per SM the registers should allow: as many as the line buffers do at
@@ -499,6 +587,7 @@ __global__ void __launch_bounds__(32 * W, sino_min_ctas(L, W, kSel))
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_range[2];
     __shared__ int s_region[4];
+    __shared__ LineShare<W / L> s_share[L];
     // support region: static, or the non-zero box found on the device
     if (threadIdx.x == 0) {
         if (a.dyn_region) {
@@ -537,7 +626,7 @@ __global__ void __launch_bounds__(32 * W, sino_min_ctas(L, W, kSel))
     for (int t = 0; t < a.n_t; t++)
         code |= (unsigned long long)(a.tf[t] & 7) << (3 * t);
     sino_block<L, kSel, kInterior, W>(J, code, a.n_t, a.need, a.stride,
-                                      reinterpret_cast<float *>(smraw), s_range);
+                                      reinterpret_cast<float *>(smraw), s_range, s_share);
 }
 
 // Persistent kernel over a batch of images of different sizes and angle
@@ -549,6 +638,7 @@ __global__ void __launch_bounds__(32 * L, sino_min_ctas(L, L, kSel))
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_range[2];
     __shared__ int s_item;
+    LineShare<1> no_share[L];
     for (;;) {
         __syncthreads(); // the previous item is done with shared memory
         if (threadIdx.x == 0)
@@ -587,7 +677,7 @@ __global__ void __launch_bounds__(32 * L, sino_min_ctas(L, L, kSel))
         J.medians = nullptr;
         J.plane = (size_t)im.n_angles * im.n;
         sino_block<L, kSel, kInterior>(J, b.tf_code, b.n_t, b.need, b.stride,
-                                       reinterpret_cast<float *>(smraw), s_range);
+                                       reinterpret_cast<float *>(smraw), s_range, no_share);
     }
 }
 
@@ -701,36 +791,6 @@ __device__ void seg_find_crossing2(const float *x, int C, float inc1, float exc1
         if (a2 && ++ln2 >= SW)
             a2 = false;
     }
-}
-
-// Eight sums over a segment of SW >= 8 lanes, transposed: three halving
-// exchanges (each lane keeps the half of the values its offset bit selects
-// and adds its partner's copy of it), then plain butterflies over the rest;
-// lane sub ends with sum k = (sub / (SW / 8)) % 8 of (a0, ..., a7).
-template <int SW>
-__device__ __forceinline__ float seg_sum8(float a0, float a1, float a2, float a3, float a4,
-                                          float a5, float a6, float a7, int sub) {
-    static_assert(SW >= 8, "eight sums need eight lanes");
-    constexpr int d1 = SW / 2, d2 = SW / 4, d3 = SW / 8;
-    bool hi = sub & d1; // keep a4..a7
-    float k0 = hi ? a4 : a0, k1 = hi ? a5 : a1, k2 = hi ? a6 : a2, k3 = hi ? a7 : a3;
-    const float s0 = hi ? a0 : a4, s1 = hi ? a1 : a5, s2 = hi ? a2 : a6, s3 = hi ? a3 : a7;
-    k0 += __shfl_xor_sync(TT_FULL_MASK, s0, d1);
-    k1 += __shfl_xor_sync(TT_FULL_MASK, s1, d1);
-    k2 += __shfl_xor_sync(TT_FULL_MASK, s2, d1);
-    k3 += __shfl_xor_sync(TT_FULL_MASK, s3, d1);
-    hi = sub & d2; // keep k2, k3
-    float m0 = hi ? k2 : k0, m1 = hi ? k3 : k1;
-    const float t0 = hi ? k0 : k2, t1 = hi ? k1 : k3;
-    m0 += __shfl_xor_sync(TT_FULL_MASK, t0, d2);
-    m1 += __shfl_xor_sync(TT_FULL_MASK, t1, d2);
-    hi = sub & d3; // keep m1
-    float r = hi ? m1 : m0;
-    r += __shfl_xor_sync(TT_FULL_MASK, hi ? m0 : m1, d3);
-#pragma unroll
-    for (int d = d3 / 2; d > 0; d >>= 1)
-        r += __shfl_xor_sync(TT_FULL_MASK, r, d);
-    return r;
 }
 
 // find_crossing_walk per segment (values of any sign).
