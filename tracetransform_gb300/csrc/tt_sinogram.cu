@@ -222,35 +222,6 @@ struct BlockJob {
 
 // ---- sampling ------------------------------------------------------------------
 
-// Two floats in one 64-bit register pair, as the packed f32x2 operations take
-// them: one issue slot for both halves.
-using pair2 = unsigned long long;
-__device__ __forceinline__ pair2 pack2(float lo, float hi) {
-    pair2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float2 unpack2(pair2 a) {
-    float2 d;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(a));
-    return d;
-}
-__device__ __forceinline__ pair2 add2_rn(pair2 a, pair2 b) {
-    pair2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ pair2 add2_rz(pair2 a, pair2 b) {
-    pair2 d;
-    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ pair2 fma2_rn(pair2 a, pair2 b, pair2 c) {
-    pair2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // Samples rows r, r + RS, ... of the rotated column `col` (row j of the frame
 // being jlo + row) into dst, zeros from row len on, dst rows < rows written.
 //
