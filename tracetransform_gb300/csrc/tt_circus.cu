@@ -344,23 +344,29 @@ __device__ __forceinline__ int stack_of(const CircusStack *st, int n_st, int v, 
 // MMA, and that rounding, not the split, bounds the error: hi.hi goes to
 // three accumulators in turn (stage s to accumulator s mod 3) and the small
 // cross terms to a fourth, so that each accumulator takes a third of the
-// big products' roundings; the epilogue adds the four in FP32.  All 256
-// threads stage the operands into shared memory in the canonical K-major
-// layout without swizzle, one block per 8-sample MMA slice: core matrices of
-// 8 rows x 16 bytes (4 samples), the slice's second 4 samples 128 bytes on
-// (LBO), the next 8 rows 256 bytes on (SBO) -- every descriptor stays inside
-// its slice's block -- into two stage buffers, each released by the commit
-// of the MMAs that read it; one thread issues a stage's 12 MMAs (4 slices x
-// 3 products).  The twiddle operand depends only on (n, frequency tile,
+// big products' roundings; the epilogue adds the four in FP32.
+//
+// Operands in shared memory, K-major, a ring of three stages.  The sinogram
+// operand: 128-byte rows (one column's 32 samples) in the 128-byte swizzle, so
+// that a warp reads 128 consecutive bytes of one column and fills one row
+// without bank conflicts (a thread per column, four samples at a time, took 32
+// sectors per load and 4096 wavefronts per stage).  The twiddle operand:
+// without swizzle, one block per 8-sample MMA slice, core matrices of 8 rows x
+// 16 bytes (4 samples), the slice's second 4 samples 128 bytes on (LBO), the
+// next 8 rows 256 bytes on (SBO).  It depends only on (n, frequency tile,
 // stage): with kPre its hi / lo blocks come precomputed in that layout
 // (p3_tc_tables_kernel) and one bulk asynchronous copy per stage brings them
-// in, completing on an mbarrier, so that the threads only split and store
-// the sinogram operand; without (the allocation-free entry point) the
-// threads gather the twiddles from the n-entry table one stage ahead.  The epilogue: warps 0-3 read their 32 lanes' accumulator rows
-// (one sinogram column per thread) and fold ck |F/n|^4 into the tile's
-// partial sum.  Every wait is bounded: a barrier that never completes (which
-// the commit protocol rules out) makes the tile's partial sums NaN instead
-// of hanging the GPU.
+// in, completing on an mbarrier; without (the allocation-free entry point) the
+// threads gather the twiddles from the n-entry table one stage ahead.  One
+// thread issues a stage's 12 MMAs (4 slices x 3 products).  The epilogue:
+// warps 0-3 read their 32 lanes' accumulator rows (one sinogram column per
+// thread) and fold ck |F/n|^4 into the tile's partial sum.  Every wait is
+// bounded: a barrier that never completes (which the commit protocol rules
+// out) makes the tile's partial sums NaN instead of hanging the GPU.
+//
+// Bound: shared-memory bandwidth -- the MMAs read 96 KB a stage and the fills
+// write 64, 1280 cycles of about 2200.  2880 columns of 1449: 105 us (116 with
+// the thread-per-column loads).
 constexpr int kTcCols = 128, kTcKT = 32, kTcThreads = 256, kTcN = 2 * kFreqTile;
 constexpr int kTcAcc = 4; // accumulators of kTcN columns: hi.hi x 3, cross terms
 constexpr int kTcAFloats = kTcCols * kTcKT, kTcBFloats = kTcN * kTcKT;
@@ -383,6 +389,13 @@ __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned 
     return (unsigned long long)((addr & 0x3ffffu) >> 4) |
            ((unsigned long long)((lbo >> 4) & 0x3fffu) << 16) |
            ((unsigned long long)((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46);
+}
+// The same for 128-byte rows in the 128-byte swizzle (8-row groups 1024 bytes
+// apart; the 16-byte chunks of row r exchanged by r mod 8), from a start
+// address inside the first row.
+__device__ __forceinline__ unsigned long long umma_desc_sw128(unsigned addr) {
+    return (unsigned long long)((addr & 0x3ffffu) >> 4) | (1ull << 16) |
+           ((unsigned long long)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 __device__ __forceinline__ void umma_tf32(unsigned d, unsigned long long a, unsigned long long b,
                                           unsigned idesc, unsigned accumulate) {
@@ -502,7 +515,7 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
         if (lane == 0) {
             const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) |
                                    ((unsigned)(N >> 3) << 17) | ((unsigned)(kTcCols >> 4) << 24);
-            const unsigned slice = kTcCols * 32; // bytes per 8-sample block (A and B: 128 rows)
+            const unsigned slice = kTcN * 32; // bytes per 8-sample block of B
             for (int s = 0; s < stages; s++) {
                 const int b = s % kTcRing;
                 ok &= mbar_wait(smem_addr(&s_full[b]), (unsigned)(s / kTcRing) & 1u);
@@ -514,8 +527,8 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
                 const unsigned dbig = tmem + (unsigned)(s % 3) * kTcN, dsmall = tmem + 3u * kTcN;
 #pragma unroll
                 for (int j = 0; j < kTcKT / 8; j++) {
-                    const unsigned long long dah = umma_desc(ahi + j * slice, 128, 256);
-                    const unsigned long long dal = umma_desc(alo + j * slice, 128, 256);
+                    const unsigned long long dah = umma_desc_sw128(ahi + j * 32);
+                    const unsigned long long dal = umma_desc_sw128(alo + j * 32);
                     const unsigned long long dbh = umma_desc(bhi + j * slice, 128, 256);
                     const unsigned long long dbl = umma_desc(blo + j * slice, 128, 256);
                     umma_tf32(dbig, dah, dbh, idesc, (s >= 3 || j > 0) ? 1u : 0u);
@@ -531,12 +544,14 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
                          : "memory");
         }
     } else {
-        // producers: column / component row r = tid & 127, sample chunks
-        // (4 samples) h, h + 2, h + 4, h + 6 of a stage, h = tid / 128
+        // producers.  Sinogram operand: warp w brings columns 16 w .. + 15, a
+        // lane one sample of the stage's 32, so that a load reads 128
+        // consecutive bytes of one column and a store fills one 128-byte row.
+        // Twiddle operand without kPre: component row r = tid & 127, sample
+        // chunks (4 samples) h, h + 2, h + 4, h + 6, h = tid / 128.
         const int r = tid & 127, h = tid >> 7;
-        const int gcol = c0 + r;
-        const float *xcol = S.sino + (size_t)min(gcol, cols - 1) * n;
-        const bool acol = gcol < cols;
+        const float *xw = S.sino + (size_t)(c0 + 16 * warp) * n + lane;
+        const int wcols = cols - c0 - 16 * warp; // of the warp's 16 that exist
         const int bf = r >> 1, be = r & 1;
         const bool brow = bf < nfreq;
         const unsigned f = (unsigned)(k0 + bf) % (unsigned)n;
@@ -544,22 +559,24 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
         unsigned idx = (f4 * (unsigned)h) % (unsigned)n; // (f p) mod n at p = p0 + 4 h
         float va[16], vb[16];
         auto fetch = [&](int p0) {
+            const bool in = p0 + lane < n;
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                va[i] = in && i < wcols ? __ldg(xw + (size_t)i * n + p0) : 0.f;
+            if (kPre)
+                return;
             unsigned ib = idx;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int kq = h + 2 * u;
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int p = p0 + 4 * kq + e;
-                    va[4 * u + e] = acol && p < n ? __ldg(xcol + p) : 0.f;
-                    if (!kPre) {
-                        float w = 0.f;
-                        if (brow && p < n) {
-                            const float2 t = __ldg(S.tw + ib);
-                            w = be ? t.y : t.x;
-                        }
-                        vb[4 * u + e] = w;
+                    float w = 0.f;
+                    if (brow && p0 + 4 * kq + e < n) {
+                        const float2 t = __ldg(S.tw + ib);
+                        w = be ? t.y : t.x;
                     }
+                    vb[4 * u + e] = w;
                     ib += f;
                     if (ib >= (unsigned)n)
                         ib -= (unsigned)n;
@@ -600,16 +617,17 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
                              : "memory");
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int kq = h + 2 * u;
-                const int off = (kq >> 1) * (kTcCols * 8) + (r >> 3) * 64 + (kq & 1) * 32 + (r & 7) * 4;
-                const float4 ah = make_float4(tf32_hi(ca[4 * u]), tf32_hi(ca[4 * u + 1]),
-                                              tf32_hi(ca[4 * u + 2]), tf32_hi(ca[4 * u + 3]));
-                *reinterpret_cast<float4 *>(Ahi + off) = ah;
-                *reinterpret_cast<float4 *>(Alo + off) =
-                    make_float4(ca[4 * u] - ah.x, ca[4 * u + 1] - ah.y, ca[4 * u + 2] - ah.z,
-                                ca[4 * u + 3] - ah.w);
-                if (!kPre) {
+            for (int i = 0; i < 16; i++) {
+                const int at = (16 * warp + i) * 32 + (lane ^ (4 * (i & 7)));
+                const float hi = tf32_hi(ca[i]);
+                Ahi[at] = hi;
+                Alo[at] = ca[i] - hi;
+            }
+            if (!kPre) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int kq = h + 2 * u;
+                    const int off = (kq >> 1) * (kTcN * 8) + (r >> 3) * 64 + (kq & 1) * 32 + (r & 7) * 4;
                     const float4 bh = make_float4(tf32_hi(cb[4 * u]), tf32_hi(cb[4 * u + 1]),
                                                   tf32_hi(cb[4 * u + 2]), tf32_hi(cb[4 * u + 3]));
                     *reinterpret_cast<float4 *>(Bhi + off) = bh;
