@@ -860,9 +860,7 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     const std::vector<const void *> key = {A, d_desc, p->nos_work.p,
                                            (const void *)(size_t)cols,
                                            (const void *)(size_t)n_sino,
-                                           (const void *)(size_t)(max_m <= 2048   ? 0
-                                                                  : max_m <= 4096 ? 1
-                                                                                  : 2)};
+                                           (const void *)(size_t)tt::nos_qr_class(max_m)};
     TT_CHECK(p->graph(p->nos_factor_graph, key, [&](cudaStream_t cs) {
         return tt::launch_nos_factor(A, d_desc, cols, n_sino, max_m, w, cs);
     }));

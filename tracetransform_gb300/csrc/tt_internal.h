@@ -228,6 +228,9 @@ cudaError_t launch_nos_align(const float *sino, int rows, int cols, int n_sino,
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
                               const NosWork &w, cudaStream_t st);
 int nos_max_rows(); // aligned rows the QR kernels hold in registers
+// Which of its kernels the QR takes for columns of up to max_m rows (a captured
+// QR serves one class).
+int nos_qr_class(int max_m);
 // One Jacobi sweep on X (n - 1 + (n & 1) launches), then the stop rule on
 // the device: the sweep sets the while-loop condition `loop` to 0 when the
 // iteration has converged or max_sweeps sweeps are done (w.sweep_state,

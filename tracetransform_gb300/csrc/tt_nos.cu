@@ -244,11 +244,16 @@ template <int T> __device__ __forceinline__ float2 qr_block_sum(float2 v, float2
 // the scalars are computed by one lane per warp.
 // At 16 rows per thread and 128 threads the next column is not prefetched:
 // that leaves 96 registers and 5 CTAs per SM instead of 128 and 4 (at
-// 8 x 1843 x 360: 4.32 against 4.50 ms for the 360 steps, same results).
+// 8 x 1843 x 360: 4.32 against 4.50 ms for the 360 steps, same results).  A
+// step is a chain over a CTA's columns, so short columns take fewer row slots
+// (K) than the 12 that 128 threads need up to 1536 rows, and with them fewer
+// registers: more CTAs per SM and fewer columns each, the same sums in the
+// same order (4 x 450 x 360: 2.11 against 2.38 ms).
+__host__ __device__ constexpr int qr_ctas(int K, int T) { // no spills below K = 32
+    return K == 32 ? 1 : T == 256 ? 2 : K == 4 ? 8 : K == 8 ? 6 : K == 12 ? 4 : 5;
+}
 template <int K, int T>
-__global__ void __launch_bounds__(T, K == 32                ? 1
-                                     : K == 16 && T == 128 ? 5
-                                                           : 512 / T) // no spills below K = 32
+__global__ void __launch_bounds__(T, qr_ctas(K, T))
 qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, int n_sino,
                int k, NosWork w) {
     constexpr int kW = T / 32;
@@ -1495,6 +1500,14 @@ static void qr_steps(float2 *A, const NosDesc *desc, int n, int n_sino, const No
 
 int nos_max_rows() { return 32 * kQrThreads; }
 
+int nos_qr_class(int max_m) {
+    const int limits[] = {4 * 128, 8 * 128, 12 * 128, 16 * 128, 16 * kQrThreads, 24 * kQrThreads};
+    int c = 0;
+    while (c < 6 && max_m > limits[c])
+        c++;
+    return c;
+}
+
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
                               const NosWork &w, cudaStream_t st) {
     if (max_m > nos_max_rows())
@@ -1502,16 +1515,28 @@ cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino,
     qr_init_kernel<<<dim3(n, n_sino), kQrThreads, 0, st>>>(A, desc, n, w);
     // 128-thread CTAs up to 2048 rows (more CTAs, and so more column chains,
     // in flight per SM), 256 above
-    if (max_m <= 12 * 128)
+    switch (nos_qr_class(max_m)) {
+    case 0:
+        qr_steps<4, 128>(A, desc, n, n_sino, w, st);
+        break;
+    case 1:
+        qr_steps<8, 128>(A, desc, n, n_sino, w, st);
+        break;
+    case 2:
         qr_steps<12, 128>(A, desc, n, n_sino, w, st);
-    else if (max_m <= 16 * 128)
+        break;
+    case 3:
         qr_steps<16, 128>(A, desc, n, n_sino, w, st);
-    else if (max_m <= 16 * kQrThreads)
+        break;
+    case 4:
         qr_steps<16, kQrThreads>(A, desc, n, n_sino, w, st);
-    else if (max_m <= 24 * kQrThreads)
+        break;
+    case 5:
         qr_steps<24, kQrThreads>(A, desc, n, n_sino, w, st);
-    else
+        break;
+    default:
         qr_steps<32, kQrThreads>(A, desc, n, n_sino, w, st);
+    }
     const long long nn = (long long)n * n;
     nos_rt_kernel<<<dim3((unsigned)((nn + 255) / 256), n_sino), 256, 0, st>>>(A, desc, n, w);
     return cudaGetLastError();
