@@ -44,8 +44,72 @@
 namespace tt {
 namespace {
 
-__global__ void nos_offsets_kernel(const float *__restrict__ sino, int rows, int n_cols,
-                                   int center, int *__restrict__ offsets) {
+// Weighted-median row - center of every column, one warp per column: the column is
+// copied to shared memory, lane 0 replaces it by its running sums in
+// the reference's order (the sum is the last of them, and the second pass's
+// integral is the first pass's running sum again), and the warp looks for the
+// first that reaches half the total.  Bound by that lane's chain of additions,
+// 4 cycles a row.  8 x 360 columns of 1449 rows: 24 us, from 197 (one thread per column
+// reading it twice, 32 cache lines per load, before).
+constexpr int kOffWarps = 4, kOffPad = 16;
+__host__ __device__ constexpr int offsets_stride(int rows) {
+    return (rows + kOffPad - 1) / kOffPad * kOffPad + kOffPad; // one block read ahead
+}
+__global__ void __launch_bounds__(32 * kOffWarps)
+nos_offsets_kernel(const float *__restrict__ sino, int rows, int n_cols, int center,
+                   int *__restrict__ offsets) {
+    extern __shared__ __align__(16) float s_off[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long idx = blockIdx.x * (long long)kOffWarps + warp;
+    if (idx >= n_cols)
+        return; // whole warps, no CTA barrier
+    const int stride = offsets_stride(rows);
+    float *x = s_off + (size_t)warp * stride;
+    const float *src = sino + (size_t)idx * rows;
+    for (int i = lane; i < stride; i += 32)
+        x[i] = i < rows ? src[i] : 0.f;
+    __syncwarp();
+    if (lane == 0) {
+        constexpr int kV = kOffPad / 4;
+        float4 *x4 = reinterpret_cast<float4 *>(x), v[kV], next[kV];
+#pragma unroll
+        for (int u = 0; u < kV; u++)
+            v[u] = x4[u];
+        float sum = 0.f;
+        for (int i = 0; i < rows; i += kOffPad, x4 += kV) {
+#pragma unroll
+            for (int u = 0; u < kV; u++)
+                next[u] = x4[kV + u];
+#pragma unroll
+            for (int u = 0; u < kV; u++) {
+                v[u].x = sum = __fadd_rn(sum, v[u].x);
+                v[u].y = sum = __fadd_rn(sum, v[u].y);
+                v[u].z = sum = __fadd_rn(sum, v[u].z);
+                v[u].w = sum = __fadd_rn(sum, v[u].w);
+                x4[u] = v[u];
+                v[u] = next[u];
+            }
+        }
+    }
+    __syncwarp();
+    const float sum = x[rows - 1];
+    int m = rows - 1;
+    for (int i0 = 0; i0 < rows; i0 += 32) {
+        const int i = i0 + lane;
+        const unsigned b = __ballot_sync(TT_FULL_MASK, i < rows && 2.f * x[min(i, rows - 1)] >= sum);
+        if (b) {
+            m = i0 + __ffs(b) - 1;
+            break;
+        }
+    }
+    if (lane == 0)
+        offsets[idx] = m - center;
+}
+
+// The same, one thread per column, for columns over nos_max_rows(): these only
+// tell how many aligned rows the call asks for, which is then refused.
+__global__ void nos_offsets_long_kernel(const float *sino, int rows, int n_cols, int center,
+                                        int *offsets) {
     const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (idx >= n_cols)
         return;
@@ -1466,8 +1530,16 @@ cudaError_t launch_nos_offsets(const float *sino, int rows, int cols, int n_sino
     const long long n = (long long)cols * n_sino;
     if (n <= 0)
         return cudaSuccess;
-    nos_offsets_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(sino, rows, (int)n, center,
-                                                                      offsets);
+    if (rows > nos_max_rows()) {
+        nos_offsets_long_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(sino, rows, (int)n,
+                                                                             center, offsets);
+        return cudaGetLastError();
+    }
+    const size_t smem = sizeof(float) * (size_t)kOffWarps * offsets_stride(rows);
+    if (smem > opt_in_smem((const void *)nos_offsets_kernel))
+        return cudaErrorInvalidValue;
+    nos_offsets_kernel<<<(unsigned)((n + kOffWarps - 1) / kOffWarps), 32 * kOffWarps, smem, st>>>(
+        sino, rows, (int)n, center, offsets);
     return cudaGetLastError();
 }
 
