@@ -170,7 +170,7 @@ struct tt_plan {
     struct Graph {
         cudaGraphExec_t exec = nullptr;
         std::vector<const void *> key;
-    } nos_factor_graph, nos_sweep_graph;
+    } nos_factor_graph[tt::kNosQrClasses], nos_sweep_graph;
     cudaStream_t capture_stream = nullptr;
     SourceTexture src;
     tt::BatchEngine *batch = nullptr;
@@ -261,9 +261,11 @@ struct tt_plan {
         for (DevBuf *b : {&in, &sino, &circ, &sig, &region, &nos, &batch_in, &batch_out, &params,
                           &nos_a, &nos_work, &nos_desc, &nos_off, &cpart, &cfb})
             cudaFree(b->p);
-        for (Graph *g : {&nos_factor_graph, &nos_sweep_graph})
-            if (g->exec)
-                cudaGraphExecDestroy(g->exec);
+        for (Graph &g : nos_factor_graph)
+            if (g.exec)
+                cudaGraphExecDestroy(g.exec);
+        if (nos_sweep_graph.exec)
+            cudaGraphExecDestroy(nos_sweep_graph.exec);
         if (capture_stream)
             cudaStreamDestroy(capture_stream);
         if (stream)
@@ -794,7 +796,7 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     TT_CUDA(cudaStreamSynchronize(st));
     desc.assign(n_sino, NosDesc{});
     centers.assign(n_sino, 0);
-    size_t a_elems = 0;
+    size_t a_elems = 0, out_elems = 0;
     int max_m = 0;
     for (int s = 0; s < n_sino; s++) {
         const int *o = off.data() + (size_t)s * cols;
@@ -804,16 +806,21 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
             return fail(TT_ERR_UNSUPPORTED,
                         "nearest orthonormal sinogram needs at least as many rows (%d) as angles "
                         "(%d)", m, cols);
-        desc[s].a_off = desc[s].out_off = (long long)a_elems;
         desc[s].m = m;
         desc[s].mx = mx;
         centers[s] = center + mx;
-        a_elems += (size_t)m * cols;
         max_m = std::max(max_m, m);
+    }
+    for (NosDesc &d : desc) {
+        d.ld = tt::nos_ld(d.m, max_m);
+        d.a_off = (long long)a_elems;
+        d.out_off = (long long)out_elems;
+        a_elems += (size_t)d.ld * cols;
+        out_elems += (size_t)d.m * cols;
     }
     TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * a_elems));
     TT_CHECK(p->ensure(p->nos_desc, sizeof(NosDesc) * n_sino));
-    TT_CHECK(p->ensure(p->nos, sizeof(float) * a_elems));
+    TT_CHECK(p->ensure(p->nos, sizeof(float) * out_elems));
     if (max_m > tt::nos_max_rows())
         return fail(TT_ERR_UNSUPPORTED,
                     "nearest orthonormal sinogram of %d aligned rows exceeds %d", max_m,
@@ -855,13 +862,16 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     const NosDesc *d_desc = (const NosDesc *)p->nos_desc.p;
     TT_CUDA(tt::launch_nos_align(d_sino, rows, cols, n_sino, d_desc, (const int *)p->nos_off.p,
                                  A, a_elems, st));
-    // QR (cols + 2 launches) and one Jacobi sweep (about cols / 16 launches),
-    // each captured once per buffer set and size and replayed
+    // QR (cols + 2 launches) and one Jacobi sweep (about cols / 12 launches),
+    // each captured once per buffer set and size and replayed.  The QR has a graph per
+    // row class, as its kernels differ: images of one size fall into
+    // several (their medians decide how many rows the alignment adds), and a
+    // capture in between costs about a millisecond.
     const std::vector<const void *> key = {A, d_desc, p->nos_work.p,
                                            (const void *)(size_t)cols,
-                                           (const void *)(size_t)n_sino,
-                                           (const void *)(size_t)tt::nos_qr_class(max_m)};
-    TT_CHECK(p->graph(p->nos_factor_graph, key, [&](cudaStream_t cs) {
+                                           (const void *)(size_t)n_sino};
+    auto &factor = p->nos_factor_graph[tt::nos_qr_class(max_m)];
+    TT_CHECK(p->graph(factor, key, [&](cudaStream_t cs) {
         return tt::launch_nos_factor(A, d_desc, cols, n_sino, max_m, w, cs);
     }));
     // the sweeps: a device-side while loop (the stop rule runs after each
@@ -870,7 +880,7 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
                             [&](cudaStream_t cs, cudaGraphConditionalHandle loop) {
                                 return tt::launch_nos_sweep(cols, n_sino, w, 40, loop, cs);
                             }));
-    TT_CUDA(cudaGraphLaunch(p->nos_factor_graph.exec, st));
+    TT_CUDA(cudaGraphLaunch(factor.exec, st));
     TT_CUDA(cudaMemsetAsync(w.sweep_state, 0, sizeof(unsigned) * 2, st));
     TT_CUDA(cudaGraphLaunch(p->nos_sweep_graph.exec, st));
     TT_CUDA(tt::launch_nos_assemble(A, d_desc, cols, n_sino, max_m, w, (float *)p->nos.p, st));

@@ -199,9 +199,10 @@ cudaError_t launch_circus_f64(const double *sino, int rows, int cols, int n_sino
 
 // Nearest orthonormal sinogram (tt_nos.cu): one aligned matrix per sinogram.
 struct NosDesc {
-    long long a_off;   // into the double-float m x cols matrices
-    long long out_off; // into the float results
+    long long a_off;   // into the double-float ld x cols matrices
+    long long out_off; // into the float m x cols results
     int m;             // rows + |max offset| + |min offset|
+    int ld;            // nos_ld(m, the call's largest m): zeros in rows m .. ld - 1
     int mx;            // max offset
 };
 // Per-call scratch of the nearest orthonormal sinogram (n = angles).
@@ -211,6 +212,7 @@ struct NosWork {
     float2 *tau, *beta, *scale; // n_sino x n each: the reflectors (double-float)
     int *cmap;                  // 2 x n_sino x n: position -> stored column, by step parity
     int *perm;                  // n_sino x n: stored column that ends at each position
+    float neg_zero = -0.f;      // the addend that keeps a packed product unfused
     float *X, *V, *P;           // n_sino x n x n each (R^T, Jacobi V, polar(R))
     float *inv;                 // n_sino x n
     unsigned *off_bits;         // n_sino: largest rotated |cos| of a sweep (float bits)
@@ -228,8 +230,12 @@ cudaError_t launch_nos_align(const float *sino, int rows, int cols, int n_sino,
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
                               const NosWork &w, cudaStream_t st);
 int nos_max_rows(); // aligned rows the QR kernels hold in registers
+// Leading dimension of an aligned matrix of m rows, max_m the call's largest: whole
+// pairs of rows for every thread of the QR's CTAs.
+int nos_ld(int m, int max_m);
 // Which of its kernels the QR takes for columns of up to max_m rows (a captured
 // QR serves one class).
+constexpr int kNosQrClasses = 7;
 int nos_qr_class(int max_m);
 // One Jacobi sweep on X (n - 1 + (n & 1) launches), then the stop rule on
 // the device: the sweep sets the while-loop condition `loop` to 0 when the

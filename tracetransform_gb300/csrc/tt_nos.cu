@@ -38,6 +38,8 @@
 // result agrees to ~3e-5 absolute (entries up to ~0.7) for condition numbers
 // up to ~1e6; Eigen's float SVD of the same matrices is far less accurate.
 // Every launch is bounded; there is no grid-wide wait.
+#include <climits>
+
 #include "tt_common.cuh"
 #include "tt_internal.h"
 
@@ -215,7 +217,7 @@ __global__ void nos_align_kernel(const float *__restrict__ sino, int rows, int c
     const NosDesc d = desc[s];
     const int shift = d.mx - offsets[(size_t)s * cols + col];
     const float *src = sino + ((size_t)s * cols + col) * rows;
-    float2 *dst = A + d.a_off + (size_t)col * d.m + shift;
+    float2 *dst = A + d.a_off + (size_t)col * d.ld + shift;
     for (int r = threadIdx.x; r < rows; r += blockDim.x)
         dst[r] = make_float2(src[r], 0.f);
 }
@@ -249,7 +251,7 @@ qr_init_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc, i
     __shared__ float2 red[kQrThreads / 32];
     const int j = blockIdx.x, s = blockIdx.y;
     const NosDesc d = desc[s];
-    const float2 *a = A + d.a_off + (size_t)j * d.m;
+    const float2 *a = A + d.a_off + (size_t)j * d.ld;
     float2 v = make_float2(0.f, 0.f);
     for (int i = threadIdx.x; i < d.m; i += kQrThreads)
         v = df_fma(a[i], a[i], v);
@@ -260,9 +262,6 @@ qr_init_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc, i
         w.cmap[(size_t)s * n + j] = j;
     }
 }
-
-// Most positions one CTA of the column step handles.
-constexpr int kQrMaxCols = 64;
 
 // Warp-then-block double-float sum through red[T / 32]; one barrier.
 // Consecutive calls must alternate between two red buffers.
@@ -281,10 +280,31 @@ template <int T> __device__ __forceinline__ float2 qr_block_sum(float2 v, float2
     return v;
 }
 
+// GB double-float warp sums in the butterfly's order (the lower lane's operand
+// first): lane g (32 / GB) ends with sum g.  Four sums share their first two
+// levels: each lane keeps the half of them that its lane bit selects.
+template <int GB> __device__ __forceinline__ float2 qr_warp_sums(float2 (&v)[GB], int lane) {
+    static_assert(GB == 1 || GB == 2 || GB == 4, "halving exchanges");
+    int o = 16;
+#pragma unroll
+    for (int h = GB / 2; h > 0; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const float2 mine = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+            const float2 got = df_shfl_xor(give, o);
+            v[i] = df_add(up ? got : mine, up ? mine : got);
+        }
+    }
+#pragma unroll
+    for (; o > 0; o >>= 1)
+        v[0] = df_add(v[0], df_shfl_xor(v[0], o));
+    return v[0];
+}
+
 // Column step k of the pivoted QR in one launch, grid (G, n_sino): CTA b
-// handles positions k + b, k + b + G, ... (G is chosen so that the grid is one
-// wave, and each CTA prefetches its next column while it reduces the current
-// one).
+// handles positions k + b, k + b + G, ... in groups of GB (G is chosen so that
+// the grid is one wave).
 //
 // Every CTA picks the pivot itself -- the remaining position of largest
 // partial norm, lowest position on ties -- and reads the pivot column
@@ -302,95 +322,119 @@ template <int T> __device__ __forceinline__ float2 qr_block_sum(float2 v, float2
 // position) and cmap are double-buffered by step parity.  perm[k] receives
 // the stored column that ends at position k.
 //
-// Element slots: thread t holds rows k + 1 + t + kQrThreads u (u < K, K kQrThreads >=
-// m) of a column in registers, so each column is read once with all loads in
-// flight and written once.  Sums, updates and scalars are all double-float;
-// the scalars are computed by one lane per warp.
-// At 16 rows per thread and 128 threads the next column is not prefetched:
-// that leaves 96 registers and 5 CTAs per SM instead of 128 and 4 (at
-// 8 x 1843 x 360: 4.32 against 4.50 ms for the 360 steps, same results).  A
-// step is a chain over a CTA's columns, so short columns take fewer row slots
-// (K) than the 12 that 128 threads need up to 1536 rows, and with them fewer
-// registers: more CTAs per SM and fewer columns each, the same sums in the
-// same order (4 x 450 x 360: 2.11 against 2.38 ms).
-__host__ __device__ constexpr int qr_ctas(int K, int T) { // no spills below K = 32
-    return K == 32 ? 1 : T == 256 ? 2 : K == 4 ? 8 : K == 8 ? 6 : K == 12 ? 4 : 5;
+// What bounds a step is the instructions issued per element, then the chain
+// map, pivot, pivot column, sums, scalars, update.  So thread t holds the row
+// pairs 2 (t + T u), u0 <= u < nu, whatever k is, in columns padded with
+// zeros to whole slots: every access is 16 bytes at a constant offset from one
+// pointer per column, and no row is tested -- x is zero up to row k, which leaves
+// the rows above untouched.  A group's columns come in by asynchronous copies
+// issued before the pivot is known, into slots of shared memory that only
+// their own thread reads (no barrier); a slot is refilled for the next group
+// once its column is written.  The sums of a whole group and |x|^2 share one
+// barrier, lane g of every warp then forms column g's scalars, and the two
+// divisions of the reflector run in two lanes.  Sums, updates and scalars
+// are all double-float.
+// The whole orthonormal circus, before (8-byte accesses, each with its own address
+// and row test, a reduction and a barrier per column) and now: 8 x 1449 x 360,
+// 9.28 and 8.3 ms; 4 x 450 x 360, 6.16 and 5.7; 8 x 5795 x 720, 90.6 and 78.8.  Two
+// rows at a time in packed operations take 40 % fewer instructions and as
+// long: a step then waits for its chain.
+//
+// K: row pairs per thread (2 K T >= ld).  CTAs per SM: by registers (four floats
+// per row pair of x, no spills) and by the slots' shared memory.  Groups of
+// two: of four, 8 x 1449 x 360 takes 8.45 against 8.31 ms in all (fewer CTAs fit);
+// of one, 8 x 5795 x 720 takes 86.9 against 78.8.
+constexpr int kQrGroup = 2;
+__host__ __device__ constexpr size_t qr_smem(int K, int T) {
+    return sizeof(float4) * (size_t)kQrGroup * K * T;
+}
+__host__ __device__ constexpr int qr_ctas(int K, int T) {
+    return T == 64 ? 10 : T == 128 ? (K == 4 ? 6 : 5) : K == 8 ? 3 : K == 12 ? 2 : 1;
 }
 template <int K, int T>
 __global__ void __launch_bounds__(T, qr_ctas(K, T))
 qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, int n_sino,
                int k, NosWork w) {
-    constexpr int kW = T / 32;
-    constexpr bool kPrefetch = K <= 12 || (K == 16 && T == 256); // registers for a second column
+    constexpr int kW = T / 32, GB = kQrGroup, kStep = 32 / GB;
+    extern __shared__ __align__(16) float4 s_slot[]; // [GB][K][T]
     __shared__ int s_bv[kW];
     __shared__ int s_bi[kW];
+    __shared__ float2 s_xn[kW];
+    __shared__ float2 s_dot[2][GB][kW];
     __shared__ float2 s_red[2][kW];
-    __shared__ float2 s_red2[kW];
-    __shared__ int s_col[kQrMaxCols];
-    __shared__ float2 s_nr[kQrMaxCols];
-    __shared__ float s_og[kQrMaxCols];
     const int s = blockIdx.y, G = gridDim.x, b = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const NosDesc d = desc[s];
-    const int m = d.m;
-    // slot (t, u) of a column holds row k + 1 + t + T u; keff slots
-    // cover the rows below the diagonal
-    const int keff = (m - k - 1 + T - 1) / T;
+    const size_t ld = d.ld;
+    // the first slot with rows below k and the slots in all
+    const int u0 = (k + 1) / (2 * T), nu = d.ld / (2 * T);
     float2 *As = A + d.a_off;
     const size_t cur = (size_t)(k & 1) * n_sino + s, nxt = (size_t)((k + 1) & 1) * n_sino + s;
     const float2 *nr = w.norms + cur * n;
     const int *cm = w.cmap + cur * n;
-    const int j0 = k + b;
-    const int cnt = min((n - j0 + G - 1) / G, kQrMaxCols);
-    // per own column: stored column, partial norm and recompute threshold
-    for (int t = threadIdx.x; t < cnt; t += T) {
-        const int c = cm[j0 + t * G];
-        s_col[t] = c;
-        s_nr[t] = nr[j0 + t * G];
-        s_og[t] = w.orig[(size_t)s * n + c];
-    }
-
-    // first own column, loaded while the pivot is chosen
-    const int c0 = cm[j0];
-    float2 cv[K];
-    {
-        const float2 *c = As + (size_t)c0 * m;
+    float *og = w.orig + (size_t)s * n;
+    const int j0 = k + b, cnt = (n - j0 + G - 1) / G;
+    const int g_mine = lane % GB;   // the group's column whose scalars this lane forms
+    float4 *slot = s_slot + threadIdx.x;
+    auto column = [&](int c) { // this thread's row pairs of column c, T apart
+        return reinterpret_cast<float4 *>(As + c * ld) + threadIdx.x;
+    };
+    auto issue = [&](int g, int c) { // column c into the slots of group member g
+        const float4 *src = column(c);
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + g * K * T);
 #pragma unroll
-        for (int u = 0; u < K; u++) {
-            const int i = k + 1 + threadIdx.x + T * u;
-            cv[u] = u < keff && i < m ? c[i] : make_float2(0.f, 0.f);
-        }
+        for (int u = 0; u < K; u++)
+            if (u >= u0 && u < nu)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 dst + (unsigned)(u * T * sizeof(float4))),
+                             "l"(src + u * T)
+                             : "memory");
+    };
+
+    // first group, on its way while the pivot is chosen
+    int c_mine = -1;     // stored column, -1 past the CTA's share
+    float2 n_mine = make_float2(0.f, 0.f), k_mine = n_mine; // partial norm and a[k]
+    float o_mine = 0.f;  // norm at the last recompute
+    if (g_mine < cnt) {
+        c_mine = cm[j0 + g_mine * G];
+        n_mine = nr[j0 + g_mine * G];
     }
-    float2 ck = As[(size_t)c0 * m + k];
+#pragma unroll
+    for (int g = 0; g < GB; g++) {
+        const int c = __shfl_sync(TT_FULL_MASK, c_mine, g);
+        if (c >= 0)
+            issue(g, c);
+    }
+    if (c_mine >= 0) {
+        k_mine = As[c_mine * ld + k];
+        o_mine = og[c_mine];
+    }
 
     // pivot: argmax of the partial norms over positions k..n-1, compared as
     // the bit patterns of their (non-negative) high words on the integer
-    // pipe; a NaN or negative norm counts as 0
-    int best = -1;
-    int bidx = n;
+    // pipe; a NaN or negative norm counts as 0.  The stored column travels with
+    // the position (n is far below 2^15).
+    int best = -1, bidx = INT_MAX;
     for (int jj = k + threadIdx.x; jj < n; jj += T) {
         int v = __float_as_int(nr[jj].x);
+        const int at = jj << 16 | cm[jj];
         if (v < 0 || v > 0x7F800000)
             v = 0;
         if (v > best) { // positions rise per thread: the first maximum stays
             best = v;
-            bidx = jj;
+            bidx = at;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int ov = __shfl_xor_sync(TT_FULL_MASK, best, o);
-        const int oi = __shfl_xor_sync(TT_FULL_MASK, bidx, o);
-        if (ov > best || (ov == best && oi < bidx)) {
-            best = ov;
-            bidx = oi;
-        }
+    {
+        const int top = __reduce_max_sync(TT_FULL_MASK, best);
+        bidx = __reduce_min_sync(TT_FULL_MASK, best == top ? bidx : INT_MAX);
+        best = top;
     }
     if (lane == 0) {
         s_bv[warp] = best;
         s_bi[warp] = bidx;
     }
-    __syncthreads(); // also publishes s_col
+    __syncthreads();
     best = s_bv[0];
     bidx = s_bi[0];
 #pragma unroll
@@ -399,156 +443,185 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
             best = s_bv[u];
             bidx = s_bi[u];
         }
-    const int p = bidx < n ? bidx : k;
-    const int cp = cm[p];
-    const float2 *x = As + (size_t)cp * m;
-    float2 xv[K];
+    const int p = bidx >> 16, cp = bidx & 0xffff;
+    const float4 *x = column(cp);
+    float4 xv[K];
 #pragma unroll
-    for (int u = 0; u < K; u++) {
-        const int i = k + 1 + threadIdx.x + T * u;
-        xv[u] = u < keff && i < m ? x[i] : make_float2(0.f, 0.f);
-    }
-    const float2 xk = x[k];
-
-    // |x[k+1:]|^2 and, for the first own column, x[k+1:] . a[k+1:]
-    float2 xn, xa;
-    {
-        DfDot dn[2], da[2];
+    for (int u = 0; u < K; u++)
+        xv[u] = u >= u0 && u < nu ? x[u * T] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 xk = As[cp * ld + k];
+    const int head = k - 2 * (int)(threadIdx.x + T * u0); // zero rows <= k of slot u0
+    if (head >= 0)
 #pragma unroll
         for (int u = 0; u < K; u++)
-            if (u < keff) {
-                df_dot_add(dn[u & 1], xv[u], xv[u]);
-                df_dot_add(da[u & 1], xv[u], cv[u]);
+            if (u == u0) {
+                xv[u].x = xv[u].y = 0.f;
+                if (head >= 1)
+                    xv[u].z = xv[u].w = 0.f;
             }
-        xn = df_add(df_dot_end(dn[0]), df_dot_end(dn[1]));
-        xa = df_add(df_dot_end(da[0]), df_dot_end(da[1]));
-    }
+    auto dot = [](DfDot (&acc)[2], float4 a, float4 c) {
+        df_dot_add(acc[0], make_float2(a.x, a.y), make_float2(c.x, c.y));
+        df_dot_add(acc[1], make_float2(a.z, a.w), make_float2(c.z, c.w));
+    };
+    {
+        DfDot dn[2];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        xn = df_add(xn, df_shfl_xor(xn, o));
-        xa = df_add(xa, df_shfl_xor(xa, o));
-    }
-    if (lane == 0) {
-        s_red[0][warp] = xn;
-        s_red2[warp] = xa;
-    }
-    __syncthreads();
-    xn = s_red[0][0];
-    xa = s_red2[0];
+        for (int u = 0; u < K; u++)
+            if (u >= u0 && u < nu)
+                dot(dn, xv[u], xv[u]);
+        float2 xn = df_add(df_dot_end(dn[0]), df_dot_end(dn[1]));
 #pragma unroll
-    for (int u = 1; u < kW; u++) {
-        xn = df_add(xn, s_red[0][u]);
-        xa = df_add(xa, s_red2[u]);
+        for (int o = 16; o > 0; o >>= 1)
+            xn = df_add(xn, df_shfl_xor(xn, o));
+        if (lane == 0)
+            s_xn[warp] = xn;
     }
-    int rb = 1; // s_red[rb] is the next free reduction buffer
-    const bool zero = xn.x == 0.f; // uniform: H = I, x stays as it is
 
-    // reflector scalars (double-float, no FP64: GB300's FP64 pipe would
-    // serialise them) by lane 0 of each warp, broadcast by shuffle
-    float2 scale_df = make_float2(0.f, 0.f), tau_df = make_float2(0.f, 0.f);
-    if (lane == 0) {
-        float2 beta = xk;
-        if (!zero) {
-            const float2 root = df_sqrt(df_fma(xk, xk, xn));
-            beta = xk.x >= 0.f ? df_neg(root) : root;
-            scale_df = df_div(make_float2(1.f, 0.f), df_sub(xk, beta));
-            tau_df = df_div(df_sub(beta, xk), beta);
-        }
-        if (warp == 0 && (p - k) % G == b) {
-            const size_t o = (size_t)s * n + k;
-            w.beta[o] = beta;
-            w.scale[o] = scale_df;
-            w.tau[o] = tau_df;
-            w.perm[o] = cp;
-        }
-    }
-    scale_df = make_float2(__shfl_sync(TT_FULL_MASK, scale_df.x, 0),
-                           __shfl_sync(TT_FULL_MASK, scale_df.y, 0));
-    tau_df = make_float2(__shfl_sync(TT_FULL_MASK, tau_df.x, 0),
-                         __shfl_sync(TT_FULL_MASK, tau_df.y, 0));
-    float *og = w.orig + (size_t)s * n;
-
-    for (int t = 0; t < cnt; t++) {
-        const int j = j0 + t * G, cj = s_col[t];
-        float2 cn[kPrefetch ? K : 1];
-        float2 ckn = make_float2(0.f, 0.f);
-        if (kPrefetch && t + 1 < cnt) {
-            const float2 *c = As + (size_t)s_col[t + 1] * m;
+    float2 scale_df = make_float2(0.f, 0.f), tau_df = scale_df;
+    bool zero = false;
+    int rb = 0, buf = 0;
+    for (int t0 = 0; t0 < cnt; t0 += GB, buf ^= 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        const int live = min(GB, cnt - t0);
+        float2 v[GB]; // x[k+1:] . a[k+1:] of the group's columns
 #pragma unroll
-            for (int u = 0; u < (kPrefetch ? K : 1); u++) {
-                const int i = k + 1 + threadIdx.x + T * u;
-                cn[u] = u < keff && i < m ? c[i] : make_float2(0.f, 0.f);
-            }
-            ckn = c[k];
-        }
-        if (j != p) { // uniform
-            float2 *c = As + (size_t)cj * m;
-            if (t > 0) {
-                DfDot dv[2];
+        for (int g = 0; g < GB; g++) {
+            DfDot dv[2];
+            if (g < live) // uniform
 #pragma unroll
                 for (int u = 0; u < K; u++)
-                    if (u < keff)
-                        df_dot_add(dv[u & 1], xv[u], cv[u]);
-                xa = qr_block_sum<T>(df_add(df_dot_end(dv[0]), df_dot_end(dv[1])), s_red[rb]);
-                rb ^= 1;
-            }
+                    if (u >= u0 && u < nu)
+                        dot(dv, xv[u], slot[(g * K + u) * T]);
+            v[g] = df_add(df_dot_end(dv[0]), df_dot_end(dv[1]));
+        }
+        const float2 part = qr_warp_sums<GB>(v, lane);
+        if (lane % kStep == 0)
+            s_dot[buf][lane / kStep][warp] = part;
+        __syncthreads();
+        if (t0 == 0) {
+            // reflector scalars (double-float, no FP64: GB300's FP64 pipe would
+            // serialise them): even lanes divide for scale, odd ones for tau
+            float2 xn = s_xn[0];
+#pragma unroll
+            for (int u = 1; u < kW; u++)
+                xn = df_add(xn, s_xn[u]);
+            zero = xn.x == 0.f; // uniform: H = I, x stays as it is
+            float2 beta = xk;
             if (!zero) {
-                // a -= tau v (v . a), v . a = a[k] + scale (x[k+1:] . a[k+1:])
-                const float2 vc = df_add(ck, df_mul(scale_df, xa));
-                const float2 ntw = df_neg(df_mul(tau_df, vc));
-                const float2 ntws = df_mul(ntw, scale_df);
-#pragma unroll
-                for (int u = 0; u < K; u++) {
-                    const int i = k + 1 + threadIdx.x + T * u;
-                    if (u < keff)
-                        cv[u] = df_fma(ntws, xv[u], cv[u]);
-                    if (u < keff && i < m)
-                        c[i] = cv[u];
-                }
-                ck = df_add(ck, ntw);
-                if (threadIdx.x == 0)
-                    c[k] = ck;
+                const float2 root = df_sqrt(df_fma(xk, xk, xn));
+                beta = xk.x >= 0.f ? df_neg(root) : root;
+                const bool tau_lane = lane & 1;
+                const float2 quot =
+                    df_div(tau_lane ? df_sub(beta, xk) : make_float2(1.f, 0.f),
+                           tau_lane ? beta : df_sub(xk, beta));
+                scale_df = make_float2(__shfl_sync(TT_FULL_MASK, quot.x, 0),
+                                       __shfl_sync(TT_FULL_MASK, quot.y, 0));
+                tau_df = make_float2(__shfl_sync(TT_FULL_MASK, quot.x, 1),
+                                     __shfl_sync(TT_FULL_MASK, quot.y, 1));
             }
-            // partial norm for step k + 1, decided by lane 0 of each warp
-            float2 n2 = make_float2(0.f, 0.f);
-            int recompute = 0;
-            if (lane == 0) {
-                n2 = df_sub(s_nr[t], df_mul(ck, ck));
-                recompute = n2.x <= 1.5e-8f * s_og[t];
-            }
-            if (__shfl_sync(TT_FULL_MASK, recompute, 0)) { // uniform
-                DfDot dr[2];
-#pragma unroll
-                for (int u = 0; u < K; u++)
-                    if (u < keff)
-                        df_dot_add(dr[u & 1], cv[u], cv[u]);
-                const float2 r = qr_block_sum<T>(df_add(df_dot_end(dr[0]), df_dot_end(dr[1])), s_red[rb]);
-                rb ^= 1;
-                n2 = r;
-                if (threadIdx.x == 0)
-                    og[cj] = n2.x;
-            }
-            if (threadIdx.x == 0) {
-                const int dest = j == k ? p : j;
-                w.norms[nxt * n + dest] = n2;
-                w.cmap[nxt * n + dest] = cj;
+            if (threadIdx.x == 0 && (p - k) % G == b) {
+                const size_t o = (size_t)s * n + k;
+                w.beta[o] = beta;
+                w.scale[o] = scale_df;
+                w.tau[o] = tau_df;
+                w.perm[o] = cp;
             }
         }
-        if (t + 1 < cnt) {
-            if (kPrefetch) {
+        // column g_mine's scalars: a -= tau v (v . a), v . a = a[k] + scale
+        // (x[k+1:] . a[k+1:]); its partial norm for step k + 1
+        const int j = j0 + (t0 + g_mine) * G;
+        const bool on = c_mine >= 0 && j != p;
+        float2 ntws = make_float2(0.f, 0.f), n2;
+        {
+            float2 xa = s_dot[buf][g_mine][0];
 #pragma unroll
-                for (int u = 0; u < (kPrefetch ? K : 1); u++)
-                    cv[u] = cn[u];
-                ck = ckn;
-            } else {
-                const float2 *c = As + (size_t)s_col[t + 1] * m;
-#pragma unroll
-                for (int u = 0; u < K; u++) {
-                    const int i = k + 1 + threadIdx.x + T * u;
-                    cv[u] = u < keff && i < m ? c[i] : make_float2(0.f, 0.f);
-                }
-                ck = c[k];
+            for (int u = 1; u < kW; u++)
+                xa = df_add(xa, s_dot[buf][g_mine][u]);
+            if (!zero) {
+                const float2 vc = df_add(k_mine, df_mul(scale_df, xa));
+                const float2 ntw = df_neg(df_mul(tau_df, vc));
+                ntws = df_mul(ntw, scale_df);
+                k_mine = df_add(k_mine, ntw);
             }
+            n2 = df_sub(n_mine, df_mul(k_mine, k_mine));
+        }
+        const bool rec = on && n2.x <= 1.5e-8f * o_mine;
+        const unsigned rec_mask = __ballot_sync(TT_FULL_MASK, rec);
+        const unsigned on_mask = __ballot_sync(TT_FULL_MASK, on);
+        // a[k] into its slot, if that is among the rewritten ones (u0 may be past it)
+        const int pair_k = (k >> 1) - T * u0;
+        const bool k_inside = pair_k >= 0;
+        if (k_inside && pair_k >> 5 == warp) {
+            if (lane < GB && on)
+                reinterpret_cast<float2 *>(s_slot + (g_mine * K + u0) * T + pair_k)[k & 1] = k_mine;
+            __syncwarp();
+        }
+        const int c_now = c_mine;
+        const float2 k_now = k_mine;
+        if (t0 + GB < cnt) { // the next group's column of this lane
+            const int tn = t0 + GB + g_mine;
+            c_mine = tn < cnt ? cm[j0 + tn * G] : -1;
+            if (c_mine >= 0) {
+                n_mine = nr[j0 + tn * G];
+                k_mine = As[c_mine * ld + k];
+                o_mine = og[c_mine];
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < GB; g++) {
+            const int cj = __shfl_sync(TT_FULL_MASK, c_now, g);
+            const float2 f = make_float2(__shfl_sync(TT_FULL_MASK, ntws.x, g),
+                                         __shfl_sync(TT_FULL_MASK, ntws.y, g));
+            if (on_mask >> g & 1) { // uniform
+                const bool again = rec_mask >> g & 1;
+                if (!zero) {
+                    float4 *c = column(cj);
+#pragma unroll
+                    for (int u = 0; u < K; u++)
+                        if (u >= u0 && u < nu) {
+                            const float4 a = slot[(g * K + u) * T], xu = xv[u];
+                            const float2 lo = df_fma(f, make_float2(xu.x, xu.y),
+                                                     make_float2(a.x, a.y));
+                            const float2 hi = df_fma(f, make_float2(xu.z, xu.w),
+                                                     make_float2(a.z, a.w));
+                            c[u * T] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                        }
+                }
+                if (again) { // rare: the norm of the new column below row k
+                    DfDot dr[2];
+                    for (int u = u0; u < nu; u++) {
+                        float4 a = slot[(g * K + u) * T];
+                        const float4 *c = column(cj);
+                        if (!zero)
+                            a = c[u * T]; // as this thread wrote it
+                        const int row = 2 * (threadIdx.x + T * u);
+                        if (row <= k)
+                            a.x = a.y = 0.f;
+                        if (row + 1 <= k)
+                            a.z = a.w = 0.f;
+                        dot(dr, a, a);
+                    }
+                    const float2 r = qr_block_sum<T>(
+                        df_add(df_dot_end(dr[0]), df_dot_end(dr[1])), s_red[rb]);
+                    rb ^= 1;
+                    if (g == g_mine)
+                        n2 = r;
+                    if (threadIdx.x == 0)
+                        og[cj] = r.x;
+                }
+            }
+            if (t0 + GB < cnt) {
+                const int c = __shfl_sync(TT_FULL_MASK, c_mine, g);
+                if (c >= 0)
+                    issue(g, c);
+            }
+        }
+        if (on && threadIdx.x < GB) {
+            if (!zero && !k_inside)
+                As[c_now * ld + k] = k_now;
+            const int dest = j == k ? p : j;
+            w.norms[nxt * n + dest] = n2;
+            w.cmap[nxt * n + dest] = c_now;
         }
     }
 }
@@ -582,7 +655,7 @@ __global__ void nos_rt_kernel(const float2 *__restrict__ A, const NosDesc *__res
     if (j == i)
         r = beta[i].x + beta[i].y;
     else if (j < i) {
-        const float2 a = A[d.a_off + j + (size_t)w.perm[(size_t)s * n + i] * d.m];
+        const float2 a = A[d.a_off + j + (size_t)w.perm[(size_t)s * n + i] * d.ld];
         r = a.x + a.y;
     }
     w.X[s * nn + e] = r;
@@ -1075,7 +1148,7 @@ nos_apply_q_reg_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__
     __syncthreads(); // scalars in place
     const float2 *As = A + d.a_off;
     auto load_v = [&](int k, float(&v)[K]) {
-        const float2 *x = As + (size_t)s_pm[k] * m;
+        const float2 *x = As + (size_t)s_pm[k] * d.ld;
         const float vs = s_vs[k];
 #pragma unroll
         for (int u = 0; u < K; u++) {
@@ -1189,14 +1262,14 @@ __device__ __forceinline__ void wy_load_refl(WyRefl &R, const float2 *tau, const
     }
 }
 // v_{k0 + r}[row] for a row inside the matrix (row < m).
-__device__ __forceinline__ float wy_v(const float2 *As, int m, const WyRefl &R, int n, int k0,
+__device__ __forceinline__ float wy_v(const float2 *As, int ld, const WyRefl &R, int n, int k0,
                                       int r, int row) {
     const int k = k0 + r;
     if (k >= n || row < k)
         return 0.f;
     if (row == k)
         return 1.f;
-    const float2 x = As[(size_t)R.pm[r] * m + row];
+    const float2 x = As[(size_t)R.pm[r] * ld + row];
     return (x.x + x.y) * R.vs[r];
 }
 
@@ -1226,7 +1299,7 @@ wy_t_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc,
         for (int q = 0; q < kPer; q++) {
             const int e = threadIdx.x + kWyThreads * q;
             const int i = e % kWyGramRows, r = e / kWyGramRows, row = row0 + i;
-            vr[q] = row < m ? wy_v(As, m, R, n, k0, r, row) : 0.f;
+            vr[q] = row < m ? wy_v(As, d.ld, R, n, k0, r, row) : 0.f;
         }
     };
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1318,7 +1391,7 @@ wy_vty_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc,
         for (int q = 0; q < kPV; q++) {
             const int e = threadIdx.x + kWyThreads * q;
             const int i = (e >> 8) * 8 + (e & 7), r = (e >> 3) & 31, row = row0 + i;
-            vr[q] = row < re ? wy_v(As, m, R, n, k0, r, row) : 0.f;
+            vr[q] = row < re ? wy_v(As, d.ld, R, n, k0, r, row) : 0.f;
         }
 #pragma unroll
         for (int q = 0; q < kPY; q++) {
@@ -1448,7 +1521,7 @@ wy_update_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc,
         for (int q = 0; q < kPV; q++) {
             const int e = threadIdx.x + kWyThreads * q;
             const int i = e & 31, r = e >> 5, row = row0 + i;
-            vr[q] = row < re ? wy_v(As, m, R, n, k0, r, row) : 0.f;
+            vr[q] = row < re ? wy_v(As, d.ld, R, n, k0, r, row) : 0.f;
         }
     };
     __syncthreads(); // R, cols and Ws in place
@@ -1554,30 +1627,52 @@ cudaError_t launch_nos_align(const float *sino, int rows, int cols, int n_sino,
 }
 
 template <int K, int T>
-static void qr_steps(float2 *A, const NosDesc *desc, int n, int n_sino, const NosWork &w,
-                     cudaStream_t st) {
-    // CTAs per sinogram: one wave over all sinograms, at most kQrMaxCols
-    // positions per CTA
+static cudaError_t qr_steps(float2 *A, const NosDesc *desc, int n, int n_sino, const NosWork &w,
+                            cudaStream_t st) {
+    // CTAs per sinogram: one wave over all sinograms
+    constexpr size_t smem = qr_smem(K, T);
+    if (smem > opt_in_smem((const void *)qr_step_kernel<K, T>))
+        return cudaErrorInvalidValue;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qr_step_kernel<K, T>, T, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qr_step_kernel<K, T>, T, smem);
     const int wave = std::max(1, sms * std::max(per_sm, 1) / std::max(n_sino, 1));
     for (int k = 0; k < n; k++) {
-        const int left = n - k;
-        const int g = std::min(left, std::max(wave, (left + kQrMaxCols - 1) / kQrMaxCols));
-        qr_step_kernel<K, T><<<dim3(g, n_sino), T, 0, st>>>(A, desc, n, n_sino, k, w);
+        // CTAs of one column while that makes at most 6 per SM, of whole groups above:
+        // the work a CTA does whatever its columns then counts for more than
+        // the chain over them (1 x 1449 x 360, 5.36 against 5.67 ms in all with
+        // groups; 4 x 450 x 360, 5.87 against 5.70)
+        const long long left = n - k;
+        const long long g =
+            left * n_sino <= 6LL * sms ? left : (left + kQrGroup - 1) / kQrGroup;
+        qr_step_kernel<K, T><<<dim3((unsigned)std::min<long long>(g, wave), n_sino), T, smem,
+                               st>>>(A, desc, n, n_sino, k, w);
     }
+    return cudaSuccess;
 }
 
 int nos_max_rows() { return 32 * kQrThreads; }
 
+// Threads per CTA and row pairs per thread of the QR by longest column: a warp
+// has about a thousand instructions a step to do whatever its columns' length,
+// so short columns take fewer warps.
+struct QrClass {
+    int threads, pairs;
+};
+constexpr QrClass kQrClasses[kNosQrClasses] = {{64, 4},  {128, 4},  {128, 6}, {128, 8},
+                                               {256, 8}, {256, 12}, {256, 16}};
+
 int nos_qr_class(int max_m) {
-    const int limits[] = {4 * 128, 8 * 128, 12 * 128, 16 * 128, 16 * kQrThreads, 24 * kQrThreads};
     int c = 0;
-    while (c < 6 && max_m > limits[c])
+    while (c < kNosQrClasses - 1 && max_m > 2 * kQrClasses[c].threads * kQrClasses[c].pairs)
         c++;
     return c;
+}
+
+int nos_ld(int m, int max_m) {
+    const int rows = 2 * kQrClasses[nos_qr_class(max_m)].threads;
+    return (m + rows - 1) / rows * rows;
 }
 
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
@@ -1585,30 +1680,31 @@ cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino,
     if (max_m > nos_max_rows())
         return cudaErrorInvalidValue;
     qr_init_kernel<<<dim3(n, n_sino), kQrThreads, 0, st>>>(A, desc, n, w);
-    // 128-thread CTAs up to 2048 rows (more CTAs, and so more column chains,
-    // in flight per SM), 256 above
+    cudaError_t e = cudaSuccess;
     switch (nos_qr_class(max_m)) {
     case 0:
-        qr_steps<4, 128>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[0].pairs, kQrClasses[0].threads>(A, desc, n, n_sino, w, st);
         break;
     case 1:
-        qr_steps<8, 128>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[1].pairs, kQrClasses[1].threads>(A, desc, n, n_sino, w, st);
         break;
     case 2:
-        qr_steps<12, 128>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[2].pairs, kQrClasses[2].threads>(A, desc, n, n_sino, w, st);
         break;
     case 3:
-        qr_steps<16, 128>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[3].pairs, kQrClasses[3].threads>(A, desc, n, n_sino, w, st);
         break;
     case 4:
-        qr_steps<16, kQrThreads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[4].pairs, kQrClasses[4].threads>(A, desc, n, n_sino, w, st);
         break;
     case 5:
-        qr_steps<24, kQrThreads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[5].pairs, kQrClasses[5].threads>(A, desc, n, n_sino, w, st);
         break;
     default:
-        qr_steps<32, kQrThreads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[6].pairs, kQrClasses[6].threads>(A, desc, n, n_sino, w, st);
     }
+    if (e != cudaSuccess)
+        return e;
     const long long nn = (long long)n * n;
     nos_rt_kernel<<<dim3((unsigned)((nn + 255) / 256), n_sino), 256, 0, st>>>(A, desc, n, w);
     return cudaGetLastError();
