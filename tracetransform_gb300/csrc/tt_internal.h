@@ -212,14 +212,14 @@ struct NosWork {
     float2 *tau, *beta, *scale; // n_sino x n each: the reflectors (double-float)
     int *cmap;                  // 2 x n_sino x n: position -> stored column, by step parity
     int *perm;                  // n_sino x n: stored column that ends at each position
-    float neg_zero = -0.f;      // the addend that keeps a packed product unfused
     float *X, *V, *P;           // n_sino x n x n each (R^T, Jacobi V, polar(R))
     float *inv;                 // n_sino x n
     unsigned *off_bits;         // n_sino: largest rotated |cos| of a sweep (float bits)
     float *tiny;                // n_sino: squared column norm below which a direction is null
     unsigned *sweep_state;      // 2: the last sweep's largest cos (float bits), sweeps done
-    float *wy;                  // nos_assemble_floats(): the blocked Q application's T
-                                // factors, partial products and T W
+    float *wy;                  // nos_assemble_floats(): the reflectors as floats, or the
+                                // blocked Q application's T factors, partial products
+                                // and T W
 };
 cudaError_t launch_nos_offsets(const float *sino, int rows, int cols, int n_sino, int center,
                                int *offsets, cudaStream_t st);

@@ -1063,45 +1063,81 @@ __global__ void rt_scale_kernel(float *__restrict__ X, const float *__restrict__
 
 // C = alpha op(A) op(B) + beta D for n x n column-major float matrices per
 // sinogram, op given by strides: op(A)(i, k) = A[i ai + k ak], op(B)(k, j) =
-// B[k bk + j bj].  32 x 32 output tiles (256 threads, 4 outputs each), k in
-// shared-memory steps of 32.  grid (ceil(n / 32), ceil(n / 32), n_sino).
+// B[k bk + j bj], one stride of each pair being 1 (the tile's loads run along
+// it).  64 x 64 output tiles, 4 x 4 per thread from two 16-byte loads per k,
+// k in steps of 16 with the next step's elements fetched meanwhile.  Three
+// products at 8 x 360^3: 96 us, from 307 (32 x 32 tiles, 4 outputs and five
+// loads per k and thread); sums in the same order.  grid (ceil(n / 64),
+// ceil(n / 64), n_sino).
+constexpr int kGemmTile = 64, kGemmStep = 16, kGemmLd = kGemmTile + 4;
 __global__ void __launch_bounds__(256)
 rt_gemm_kernel(const float *__restrict__ A, int ai, int ak, const float *__restrict__ B, int bk,
                int bj, const float *__restrict__ D, float alpha, float beta, int n,
                float *__restrict__ C) {
-    __shared__ float as[32][33], bs[32][33];
-    const int ti = threadIdx.x & 31, tj = threadIdx.x >> 5; // tj 0..7
-    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+    __shared__ __align__(16) float as[kGemmStep][kGemmLd], bs[kGemmStep][kGemmLd];
+    const int i0 = blockIdx.x * kGemmTile, j0 = blockIdx.y * kGemmTile;
+    const int ti = 4 * (threadIdx.x & 15), tj = 4 * (threadIdx.x >> 4);
     const size_t off = (size_t)blockIdx.z * n * n;
     A += off;
     B += off;
     C += off;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k0 = 0; k0 < n; k0 += 32) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < 32 * 32; e += 256) {
-            const int r = e & 31, kk = e >> 5, k = k0 + kk;
-            as[kk][r] = (k < n && i0 + r < n) ? A[(size_t)(i0 + r) * ai + (size_t)k * ak] : 0.f;
-            bs[kk][r] = (k < n && j0 + r < n) ? B[(size_t)k * bk + (size_t)(j0 + r) * bj] : 0.f;
+    // this thread's four elements of a step: (row of the tile, k) of each operand
+    constexpr int kPer = kGemmTile * kGemmStep / 256;
+    auto place = [](bool along_k, int q, int &r, int &kk) {
+        const int e = threadIdx.x + 256 * q;
+        r = along_k ? e / kGemmStep : e % kGemmTile;
+        kk = along_k ? e % kGemmStep : e / kGemmTile;
+    };
+    float an[kPer], bn[kPer];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            int r, kk;
+            place(ak == 1, q, r, kk);
+            an[q] = k0 + kk < n && i0 + r < n ? A[(size_t)(i0 + r) * ai + (size_t)(k0 + kk) * ak]
+                                              : 0.f;
+            place(bk == 1, q, r, kk);
+            bn[q] = k0 + kk < n && j0 + r < n ? B[(size_t)(k0 + kk) * bk + (size_t)(j0 + r) * bj]
+                                              : 0.f;
+        }
+    };
+    float acc[4][4] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < n; k0 += kGemmStep) {
+        __syncthreads(); // the last step's tiles are read
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            int r, kk;
+            place(ak == 1, q, r, kk);
+            as[kk][r] = an[q];
+            place(bk == 1, q, r, kk);
+            bs[kk][r] = bn[q];
         }
         __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < 32; kk++) {
-            const float a = as[kk][ti];
+        if (k0 + kGemmStep < n)
+            fetch(k0 + kGemmStep);
+#pragma unroll
+        for (int kk = 0; kk < kGemmStep; kk++) {
+            const float4 a = *reinterpret_cast<const float4 *>(&as[kk][ti]);
+            const float4 b = *reinterpret_cast<const float4 *>(&bs[kk][tj]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                acc[u] = fmaf(a, bs[kk][tj + 8 * u], acc[u]);
-        }
-    }
-    const int i = i0 + ti;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int j = j0 + tj + 8 * u;
-        if (i < n && j < n) {
-            const size_t e = i + (size_t)j * n;
-            C[e] = beta != 0.f ? alpha * acc[u] + beta * D[off + e] : alpha * acc[u];
+                for (int v = 0; v < 4; v++)
+                    acc[u][v] = fmaf(av[u], bv[v], acc[u][v]);
         }
     }
+#pragma unroll
+    for (int v = 0; v < 4; v++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = i0 + ti + u, j = j0 + tj + v;
+            if (i < n && j < n) {
+                const size_t e = i + (size_t)j * n;
+                C[e] = beta != 0.f ? alpha * acc[u][v] + beta * D[off + e] : alpha * acc[u][v];
+            }
+        }
 }
 
 // Y = Q [P; 0] = H_0 H_1 ... H_{n-1} [P; 0], out[:, perm[j]] = Y[:, j]:
@@ -1110,32 +1146,54 @@ rt_gemm_kernel(const float *__restrict__ A, int ai, int ak, const float *__restr
 constexpr int kQThreads = 256, kQCols = 4; // columns of Y per CTA
 constexpr int kNosMaxCols = 1024;              // angles the orthonormal circus takes
 
+// The reflectors as floats, in their order: refl[s][k][i] = 1 at i = k, the scaled
+// pivot column below it, 0 above and in the rows past m, reflector stride ldv (a
+// multiple of kQThreads).  grid (n, n_sino).
+__global__ void __launch_bounds__(kQThreads)
+nos_refl_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc,
+                const float2 *__restrict__ scale, const int *__restrict__ perm, int n, int ldv,
+                float *__restrict__ refl) {
+    const int k = blockIdx.x, s = blockIdx.y;
+    const NosDesc d = desc[s];
+    const float2 sc = scale[(size_t)s * n + k];
+    const float vs = sc.x + sc.y;
+    const float2 *x = A + d.a_off + (size_t)perm[(size_t)s * n + k] * d.ld;
+    float *v = refl + ((size_t)s * n + k) * ldv;
+    for (int i = threadIdx.x; i < ldv; i += kQThreads) {
+        float vi = i == k ? 1.f : 0.f;
+        if (i > k && i < d.m) {
+            const float2 xi = x[i];
+            vi = (xi.x + xi.y) * vs;
+        }
+        v[i] = vi;
+    }
+}
+
 // The product with Y held in registers, for m <= K kQThreads: thread t
 // owns rows t + kQThreads u (u < K) of the kQCols columns, so applying a
 // reflector needs one block reduction (double-buffered: one barrier) and no
-// other exchange; the next reflector's column is loaded while the current
-// one is applied, and the reflector scalars sit in shared memory.  Slot
-// (t, u) of reflector k holds v_i for i = t + kQThreads u: 1 at i = k, the
-// scaled pivot column below it, 0 above.
+// other exchange; the next reflector is loaded while the current one is applied.
+// Bound by its instructions: the reflectors are formed once, not by every
+// CTA, and the four columns' warp sums share their first two levels.  8 x 1843 x
+// 360: 463 us, from 723; the same sums.
 template <int K>
 __global__ void __launch_bounds__(kQThreads, K == 8 ? 3 : 1) // 3 CTAs per SM fit K = 8 unspilled
-nos_apply_q_reg_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__ desc,
-                       const float2 *__restrict__ tau, const float2 *__restrict__ scale,
+nos_apply_q_reg_kernel(const float *__restrict__ refl, int ldv,
+                       const NosDesc *__restrict__ desc, const float2 *__restrict__ tau,
                        const int *__restrict__ perm, const float *__restrict__ P, int n,
                        float *__restrict__ out) {
-    __shared__ float s_t[kNosMaxCols], s_vs[kNosMaxCols];
-    __shared__ int s_pm[kNosMaxCols];
-    __shared__ float red[2][kQThreads / 32][kQCols];
+    static_assert(kQCols == 4, "the halving exchanges below");
+    __shared__ float s_t[kNosMaxCols];
+    __shared__ __align__(16) float red[2][kQThreads / 32][kQCols];
     const int s = blockIdx.y, j0 = blockIdx.x * kQCols;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const NosDesc d = desc[s];
     const int m = d.m, nc = min(kQCols, n - j0);
+    const int nu = (m + kQThreads - 1) / kQThreads; // row slots in use
     const size_t nn = (size_t)n * n;
     for (int k = threadIdx.x; k < n; k += kQThreads) {
-        const float2 t = tau[(size_t)s * n + k], v = scale[(size_t)s * n + k];
+        const float2 t = tau[(size_t)s * n + k];
         s_t[k] = t.x + t.y;
-        s_vs[k] = v.x + v.y;
-        s_pm[k] = perm[(size_t)s * n + k];
     }
     float y[kQCols][K];
 #pragma unroll
@@ -1146,29 +1204,19 @@ nos_apply_q_reg_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__
             y[c][u] = (c < nc && i < n) ? P[s * nn + i + (size_t)(j0 + c) * n] : 0.f;
     }
     __syncthreads(); // scalars in place
-    const float2 *As = A + d.a_off;
-    auto load_v = [&](int k, float(&v)[K]) {
-        const float2 *x = As + (size_t)s_pm[k] * d.ld;
-        const float vs = s_vs[k];
-#pragma unroll
-        for (int u = 0; u < K; u++) {
-            const int i = threadIdx.x + kQThreads * u;
-            float vi = 0.f;
-            if (i > k && i < m) {
-                const float2 xi = x[i];
-                vi = (xi.x + xi.y) * vs;
-            } else if (i == k) {
-                vi = 1.f;
-            }
-            v[u] = vi;
-        }
-    };
+    const float *vp = refl + ((size_t)s * n + n - 1) * ldv + threadIdx.x;
     float v[K], vn[K];
-    load_v(n - 1, v);
+#pragma unroll
+    for (int u = 0; u < K; u++)
+        v[u] = vn[u] = u < nu ? vp[kQThreads * u] : 0.f;
     int rb = 0;
     for (int k = n - 1; k >= 0; k--) {
+        vp -= ldv;
         if (k > 0)
-            load_v(k - 1, vn);
+#pragma unroll
+            for (int u = 0; u < K; u++)
+                if (u < nu)
+                    vn[u] = vp[kQThreads * u];
         const float t = s_t[k];
         if (t != 0.f) { // uniform
             float w[kQCols];
@@ -1178,21 +1226,36 @@ nos_apply_q_reg_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__
 #pragma unroll
                 for (int u = 0; u < K; u++)
                     w[c] = fmaf(v[u], y[c][u], w[c]);
-                w[c] = warp_sum(w[c]);
             }
-            if (lane == 0)
+            // lane 8 c ends with the warp's sum of column c
+            {
+                const bool up = lane & 16;
+                const float g0 = up ? w[0] : w[2], g1 = up ? w[1] : w[3];
+                float a0 = (up ? w[2] : w[0]) + __shfl_xor_sync(TT_FULL_MASK, g0, 16);
+                const float a1 = (up ? w[3] : w[1]) + __shfl_xor_sync(TT_FULL_MASK, g1, 16);
+                const bool odd = lane & 8;
+                const float g = odd ? a0 : a1;
+                a0 = (odd ? a1 : a0) + __shfl_xor_sync(TT_FULL_MASK, g, 8);
 #pragma unroll
-                for (int c = 0; c < kQCols; c++)
-                    red[rb][warp][c] = w[c];
+                for (int o = 4; o > 0; o >>= 1)
+                    a0 += __shfl_xor_sync(TT_FULL_MASK, a0, o);
+                if ((lane & 7) == 0)
+                    red[rb][warp][lane >> 3] = a0;
+            }
             __syncthreads();
+            float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int c = 0; c < kQCols; c++) {
-                float tot = 0.f;
-#pragma unroll
-                for (int q = 0; q < kQThreads / 32; q++)
-                    tot += red[rb][q][c];
-                w[c] = t * tot;
+            for (int q = 0; q < kQThreads / 32; q++) {
+                const float4 r = *reinterpret_cast<const float4 *>(red[rb][q]);
+                tot.x += r.x;
+                tot.y += r.y;
+                tot.z += r.z;
+                tot.w += r.w;
             }
+            w[0] = t * tot.x;
+            w[1] = t * tot.y;
+            w[2] = t * tot.z;
+            w[3] = t * tot.w;
             rb ^= 1;
 #pragma unroll
             for (int u = 0; u < K; u++)
@@ -1205,7 +1268,7 @@ nos_apply_q_reg_kernel(const float2 *__restrict__ A, const NosDesc *__restrict__
             v[u] = vn[u];
     }
     for (int c = 0; c < nc; c++) {
-        float *o = out + d.out_off + (size_t)s_pm[j0 + c] * m;
+        float *o = out + d.out_off + (size_t)perm[(size_t)s * n + j0 + c] * m;
 #pragma unroll
         for (int u = 0; u < K; u++) {
             const int i = threadIdx.x + kQThreads * u;
@@ -1778,12 +1841,14 @@ static WyShape wy_shape(int n, int n_sino, int max_m) {
 // aligned columns no longer fit its registers (measured on 8 sinograms of
 // 5795 x 720: the whole assembly 9.5 ms against 32.4 ms with a shared-memory
 // form of the one-reflector-at-a-time kernel; on 1843 x 360 the register
-// kernel is the faster, 1.04 against 1.33 ms).
+// kernel is the faster: 1.04 against 1.33 ms, and 0.6 since).
 static bool wy_path(int n, int max_m) { return n > kNosMaxCols || max_m > 16 * kQThreads; }
+
+static int nos_refl_ld(int max_m) { return (max_m + kQThreads - 1) / kQThreads * kQThreads; }
 
 size_t nos_assemble_floats(int n, int n_sino, int max_m) {
     if (!wy_path(n, max_m))
-        return 0;
+        return (size_t)n_sino * n * nos_refl_ld(max_m);
     const WyShape w = wy_shape(n, n_sino, max_m);
     return w.t_floats + w.part_floats + w.w2_floats;
 }
@@ -1791,7 +1856,7 @@ size_t nos_assemble_floats(int n, int n_sino, int max_m) {
 cudaError_t launch_nos_assemble(const float2 *A, const NosDesc *desc, int n, int n_sino,
                                 int max_m, const NosWork &w, float *out, cudaStream_t st) {
     const long long nn = (long long)n * n;
-    const dim3 ge((unsigned)((nn + 255) / 256), n_sino), gt((n + 31) / 32, (n + 31) / 32, n_sino);
+    const dim3 ge((unsigned)((nn + 255) / 256), n_sino), gt((n + kGemmTile - 1) / kGemmTile, (n + kGemmTile - 1) / kGemmTile, n_sino);
     rt_invnorm_kernel<<<dim3((n + 3) / 4, n_sino), 128, 0, st>>>(w.X, n, w.tiny, w.inv);
     rt_scale_kernel<<<ge, 256, 0, st>>>(w.X, w.inv, n);
     // P = V U^T, then one Newton-Schulz step P <- P (3 I - P^T P) / 2 (in the
@@ -1802,14 +1867,16 @@ cudaError_t launch_nos_assemble(const float2 *A, const NosDesc *desc, int n, int
     rt_gemm_kernel<<<gt, 256, 0, st>>>(w.P, n, 1, w.P, 1, n, nullptr, 1.f, 0.f, n, w.X);
     rt_gemm_kernel<<<gt, 256, 0, st>>>(w.P, 1, n, w.X, 1, n, w.P, -0.5f, 1.5f, n, w.V);
     const dim3 gq((n + kQCols - 1) / kQCols, n_sino);
-    if (!wy_path(n, max_m) && max_m <= 8 * kQThreads) {
-        nos_apply_q_reg_kernel<8><<<gq, kQThreads, 0, st>>>(A, desc, w.tau, w.scale, w.perm,
-                                                             w.V, n, out);
-        return cudaGetLastError();
-    }
     if (!wy_path(n, max_m)) {
-        nos_apply_q_reg_kernel<16><<<gq, kQThreads, 0, st>>>(A, desc, w.tau, w.scale, w.perm,
-                                                              w.V, n, out);
+        const int ldv = nos_refl_ld(max_m);
+        nos_refl_kernel<<<dim3(n, n_sino), kQThreads, 0, st>>>(A, desc, w.scale, w.perm, n, ldv,
+                                                                w.wy);
+        if (max_m <= 8 * kQThreads)
+            nos_apply_q_reg_kernel<8><<<gq, kQThreads, 0, st>>>(w.wy, ldv, desc, w.tau, w.perm,
+                                                                 w.V, n, out);
+        else
+            nos_apply_q_reg_kernel<16><<<gq, kQThreads, 0, st>>>(w.wy, ldv, desc, w.tau, w.perm,
+                                                                  w.V, n, out);
         return cudaGetLastError();
     }
     // Y = Q [P; 0] in the output, block by block (last block first)
