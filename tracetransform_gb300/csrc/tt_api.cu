@@ -171,7 +171,8 @@ struct tt_plan {
         cudaGraphExec_t exec = nullptr;
         std::vector<const void *> key;
     } nos_factor_graph[tt::kNosQrClasses], nos_sweep_graph;
-    cudaStream_t capture_stream = nullptr;
+    cudaStream_t capture_stream = nullptr, capture_side = nullptr; // and a branch beside it
+    cudaEvent_t capture_fork = nullptr, capture_join = nullptr;
     SourceTexture src;
     tt::BatchEngine *batch = nullptr;
     // backward / double-precision tables
@@ -266,8 +267,12 @@ struct tt_plan {
                 cudaGraphExecDestroy(g.exec);
         if (nos_sweep_graph.exec)
             cudaGraphExecDestroy(nos_sweep_graph.exec);
-        if (capture_stream)
-            cudaStreamDestroy(capture_stream);
+        for (cudaStream_t cs : {capture_stream, capture_side})
+            if (cs)
+                cudaStreamDestroy(cs);
+        for (cudaEvent_t ev : {capture_fork, capture_join})
+            if (ev)
+                cudaEventDestroy(ev);
         if (stream)
             cudaStreamDestroy(stream);
         cudaSetDevice(prev);
@@ -318,6 +323,11 @@ struct tt_plan {
         }
         if (!capture_stream)
             TT_CUDA(cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking));
+        if (!capture_side)
+            TT_CUDA(cudaStreamCreateWithFlags(&capture_side, cudaStreamNonBlocking));
+        for (cudaEvent_t *ev : {&capture_fork, &capture_join})
+            if (!*ev)
+                TT_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
         cudaGraph_t gr = nullptr;
         TT_CUDA(cudaGraphCreate(&gr, 0));
         cudaGraphConditionalHandle loop = 0;
@@ -829,14 +839,16 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
         return fail(TT_ERR_UNSUPPORTED, "orthonormal circus of %d angles exceeds 1024", cols);
     // scratch: 5 double-float + 3 int vectors of n, 3 float n x n matrices,
     // 2 float vectors, the sweep loop's state, then (256-byte aligned) the
-    // blocked Q application's
+    // sweeps' rotations and the Q application's
     const size_t nv = ncol, nm = (size_t)cols * cols * n_sino;
     const size_t head = sizeof(float2) * 5 * nv + sizeof(int) * 3 * nv +
                         sizeof(float) * (3 * nm + 2 * nv) + sizeof(unsigned) * n_sino +
                         sizeof(float) * n_sino + sizeof(unsigned) * 2;
     const size_t wy_at = (head + 255) & ~size_t(255);
+    const size_t rotations = tt::nos_rotation_floats(cols, n_sino); // a multiple of 64
     TT_CHECK(p->ensure(p->nos_work,
-                       wy_at + sizeof(float) * tt::nos_assemble_floats(cols, n_sino, max_m)));
+                       wy_at + sizeof(float) * (rotations +
+                                                tt::nos_assemble_floats(cols, n_sino, max_m))));
     tt::NosWork w;
     {
         char *q = (char *)p->nos_work.p;
@@ -854,7 +866,8 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
         w.off_bits = (unsigned *)(w.perm + nv);
         w.tiny = (float *)(w.off_bits + n_sino);
         w.sweep_state = (unsigned *)(w.tiny + n_sino);
-        w.wy = (float *)((char *)p->nos_work.p + wy_at);
+        w.J = (float *)((char *)p->nos_work.p + wy_at);
+        w.wy = w.J + rotations;
     }
     TT_CUDA(cudaMemcpyAsync(p->nos_desc.p, desc.data(), sizeof(NosDesc) * n_sino,
                             cudaMemcpyHostToDevice, st));
@@ -878,7 +891,9 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     // sweep on the device), at most 40
     TT_CHECK(p->while_graph(p->nos_sweep_graph, key,
                             [&](cudaStream_t cs, cudaGraphConditionalHandle loop) {
-                                return tt::launch_nos_sweep(cols, n_sino, w, 40, loop, cs);
+                                return tt::launch_nos_sweep(cols, n_sino, w, 40, loop, cs,
+                                                            p->capture_side, p->capture_fork,
+                                                            p->capture_join);
                             }));
     TT_CUDA(cudaGraphLaunch(factor.exec, st));
     TT_CUDA(cudaMemsetAsync(w.sweep_state, 0, sizeof(unsigned) * 2, st));

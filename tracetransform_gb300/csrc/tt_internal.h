@@ -213,6 +213,7 @@ struct NosWork {
     int *cmap;                  // 2 x n_sino x n: position -> stored column, by step parity
     int *perm;                  // n_sino x n: stored column that ends at each position
     float *X, *V, *P;           // n_sino x n x n each (R^T, Jacobi V, polar(R))
+    float *J;                   // nos_rotation_floats(): two sweeps' block rotations
     float *inv;                 // n_sino x n
     unsigned *off_bits;         // n_sino: largest rotated |cos| of a sweep (float bits)
     float *tiny;                // n_sino: squared column norm below which a direction is null
@@ -241,8 +242,11 @@ int nos_qr_class(int max_m);
 // the device: the sweep sets the while-loop condition `loop` to 0 when the
 // iteration has converged or max_sweeps sweeps are done (w.sweep_state,
 // zeroed before the loop, counts them).
+// V's rotations run on `side`, forked from and joined to st by the events.
 cudaError_t launch_nos_sweep(int n, int n_sino, const NosWork &w, int max_sweeps,
-                             cudaGraphConditionalHandle loop, cudaStream_t st);
+                             cudaGraphConditionalHandle loop, cudaStream_t st, cudaStream_t side,
+                             cudaEvent_t fork, cudaEvent_t join);
+size_t nos_rotation_floats(int n, int n_sino);
 // Scratch floats (NosWork.wy) of launch_nos_assemble.
 size_t nos_assemble_floats(int n, int n_sino, int max_m);
 // The nearest orthonormal sinograms from the converged sweeps:

@@ -24,8 +24,8 @@
 //   Jacobi        one-sided Jacobi on X = R^T in float (R^T of a pivoted QR is
 //                 graded, so float rotations keep relative accuracy), block-
 //                 cyclic: round-robin rounds of 12-column block pairs, each
-//                 pair rotated in one CTA's shared memory with V updated once
-//                 per round through the accumulated rotation;
+//                 pair rotated in one CTA's shared memory; V follows a
+//                 sweep behind through the rounds' accumulated rotations;
 //                 X V = U_X S, so polar(R) = V U_X^T
 //   assemble      P = V U_X^T (float) with one Newton-Schulz step to clean
 //                 its orthogonality, then polar(A P) = Q [P; 0] applied
@@ -681,19 +681,17 @@ constexpr float kJacTol = 1e-6f, kJacDone = 1e-4f;
 // inside each of its two blocks (kBJ - 1 more inner rounds).  A block-cyclic
 // ordering of the cyclic Jacobi method.
 //
-// V does not take part in the inner rounds: their rotations are accumulated
-// into a 2 kBJ x 2 kBJ orthogonal J (in shared memory), and the block's
-// columns of V are multiplied by J once per round, in row chunks staged
-// through shared memory.  Columns sit in shared memory zero-padded to a
+// V does not take part in the rounds: a round's rotations are accumulated into
+// one 2 kBJ x 2 kBJ orthogonal J per block pair (in shared memory), which
+// goes to global memory, and a whole sweep of them is applied to V by another
+// kernel (jacobi_v_kernel) beside the next sweep's rounds.  Columns sit in shared memory zero-padded to a
 // multiple of 128 rows, so a lane moves 4 consecutive rows per 128-bit
 // access and no row needs a bounds test.  Blocks of 12 (measured at 8
 // sinograms of 1449 x 360 and 5795 x 720: 11 % and 29 % faster sweeps than
 // blocks of 16, whose inner rounds are longer; blocks of 8 took one sweep
 // more) give a round of 8 x 360-angle sinograms 120 CTAs.
 constexpr int kBJ = 12, kBCols = 2 * kBJ, kBThreads = 32 * kBJ;
-constexpr int kVRows = 256; // rows of V per chunk: 64 groups of 4 rows x kBCols / 4 of 4 columns
 static_assert(kBJ % 2 == 0 && kBCols <= 32, "whole pairs per block; a J row per lane");
-static_assert(kBThreads == (kVRows / 4) * (kBCols / 4), "one 4 x 4 tile of V J per thread");
 
 __device__ __forceinline__ void round_robin(int players, int round, int k, int &p, int &q) {
     const int P1 = players - 1;
@@ -711,18 +709,14 @@ __device__ __forceinline__ void round_robin(int players, int round, int k, int &
     }
 }
 
-// The V block sits whole in shared memory up to 4 slots of 128 rows; larger
-// ones go through a kVRows chunk.
-__host__ __device__ constexpr bool block_round_whole_v(int k4) { return k4 <= 4; }
-
 // Dynamic shared memory of the round kernel with K4 slots of 128 rows
-// (floats): the X block, the V block (or chunk, leading dimension rows + 4)
-// and the two copies of J.
+// (floats): the X block and J.
 __host__ __device__ constexpr size_t block_round_smem_floats(int k4) {
-    return (size_t)kBCols * 128 * k4 +
-           (size_t)kBCols * ((block_round_whole_v(k4) ? 128 * k4 : kVRows) + 4) +
-           kBCols * (kBCols + 1) + kBCols * kBCols;
+    return (size_t)kBCols * 128 * k4 + kBCols * (kBCols + 1);
 }
+
+// Floats of a block pair's J, row-major; a sweep holds one per round and pair.
+constexpr int kBJFloats = kBCols * kBCols;
 
 __device__ __forceinline__ float4 f4_lin(float a, float4 x, float b, float4 y) {
     return make_float4(a * x.x + b * y.x, a * x.y + b * y.y, a * x.z + b * y.z, a * x.w + b * y.w);
@@ -866,17 +860,13 @@ __device__ __forceinline__ float jacobi_pair(float4 (&x)[K4], float4 (&y)[K4], f
 // 4 l + 128 u .. + 3 (u < K4) of a column.
 template <int K4>
 __global__ void __launch_bounds__(kBThreads)
-rt_block_round_kernel(float *__restrict__ X, float *__restrict__ V, int n, int nbp, int round,
-                      unsigned *__restrict__ off_bits, const float *__restrict__ tiny) {
+rt_block_round_kernel(float *__restrict__ X, float *__restrict__ J, int n, int nbp, int round,
+                      unsigned *__restrict__ off_bits, const float *__restrict__ tiny,
+                      const unsigned *__restrict__ state) {
     extern __shared__ __align__(16) float bsm[];
     constexpr int NP = 128 * K4; // padded rows
-    constexpr bool kWholeV = block_round_whole_v(K4);
-    constexpr int VR = kWholeV ? NP : kVRows; // rows of the V buffer
-    constexpr int VLD = VR + 4;               // its leading dimension (bank spread)
-    float *Xl = bsm;                          // kBCols x NP
-    float *Vb = Xl + (size_t)kBCols * NP;     // kBCols x VLD
-    float(*Jt)[kBCols + 1] = reinterpret_cast<float(*)[kBCols + 1]>(Vb + kBCols * VLD);
-    float(*Jr)[kBCols] = reinterpret_cast<float(*)[kBCols]>(&Jt[kBCols][0]); // row-major J
+    float *Xl = bsm;             // kBCols x NP
+    float(*Jt)[kBCols + 1] = reinterpret_cast<float(*)[kBCols + 1]>(Xl + (size_t)kBCols * NP);
     const int s = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (n + kBJ - 1) / kBJ;
     int bp, bq;
@@ -885,18 +875,16 @@ rt_block_round_kernel(float *__restrict__ X, float *__restrict__ V, int n, int n
     if (bq >= nb && !intra)
         return; // the bye (the dummy block's columns are zeros and never rotate)
     const size_t nn = (size_t)n * n;
-    float *Xg = X + s * nn, *Vg = V + s * nn;
+    float *Xg = X + s * nn;
     // global column of local column c
     auto gcol = [&](int c) { return c < kBJ ? bp * kBJ + c : bq * kBJ + c - kBJ; };
-    // X block (zero-padded to NP rows), then -- in flight during the inner
-    // rounds -- the V block (or its first chunk); J = I
+    // X block (zero-padded to NP rows); J = I
     stage_cols_async(Xl, NP, Xg, n, 0, NP, gcol);
-    cp_async_commit();
-    stage_cols_async(Vb, VLD, Vg, n, 0, VR, gcol);
     cp_async_commit();
     for (int e = threadIdx.x; e < kBCols * kBCols; e += kBThreads)
         Jt[e / kBCols][e % kBCols] = e / kBCols == e % kBCols ? 1.f : 0.f;
-    cp_async_wait<1>();
+    const unsigned parity = state[1] & 1; // of the sweep: which half of J
+    cp_async_wait<0>();
     __syncthreads();
     const float tn = tiny[s];
     float wmax = 0.f;
@@ -969,69 +957,117 @@ rt_block_round_kernel(float *__restrict__ X, float *__restrict__ V, int n, int n
         atomicMax(off_bits + s, __float_as_uint(wmax));
     // X block back
     store_cols(Xg, Xl, NP, n, 0, NP, gcol);
-    for (int e = threadIdx.x; e < kBCols * kBCols; e += kBThreads)
-        Jr[e / kBCols][e % kBCols] = Jt[e % kBCols][e / kBCols];
+    const size_t pair =
+        (((size_t)parity * gridDim.y + s) * (nbp - 1) + round) * (nbp / 2) + blockIdx.x;
+    float *Jg = J + pair * kBJFloats;
+    for (int e = threadIdx.x; e < kBJFloats; e += kBThreads)
+        Jg[e] = Jt[e % kBCols][e / kBCols];
+}
 
-    // V block <- V block J, kVRows rows per pass: thread t computes rows
-    // 4 (t / G) .. + 3 and columns 4 (t % G) .. + 3 of each pass, G = kBCols / 4
-    constexpr int kCG = kBCols / 4;
-    const int cg = (threadIdx.x % kCG) * 4, rg = (threadIdx.x / kCG) * 4;
-    auto vj_tile = [&](const float *vb, int ld, float (&acc)[4][4]) {
+// V <- V J_0 J_1 ... : the last finished sweep's rotations, round by round, applied
+// to the rows of V, which are independent: a warp keeps 4 rows (all columns, in
+// shared memory) for the whole sweep.  Per round a lane takes tiles of 4 rows x
+// 4 columns of a block pair, 24 steps of two 16-byte loads and 16
+// multiply-adds; the CTA's warps share the J's, staged 16 pairs (3 tiles
+// per lane) ahead.  Runs beside the next sweep's rounds, which are chains that leave
+// most of the machine idle.  Orthonormal circus with V rotated inside the rounds, and
+// so: 4 x 450 x 360, 5.56 and 4.97 ms; 8 x 1449 x 360, 8.04 and 7.79; 8 x 5795 x 720,
+// 77.3 and 76.7.  Keeping the rounds' CTAs off its SMs (one CTA with all the shared
+// memory on each SM they leave) measured slower, 7.85 at 8 x 1449 x 360.
+// grid (ceil(n / (4 warps)), n_sino).
+constexpr int kVMaxWarps = 8, kVPairs = 16, kVPairLd = kBJFloats + 24; // pairs 24 banks apart
+constexpr int kVTiles = kVPairs * (kBCols / 4) / 32;
+static_assert(kVTiles * 32 == kVPairs * (kBCols / 4), "whole tiles per lane");
+constexpr size_t jacobi_v_smem(int nbp, int warps) {
+    return sizeof(float) * ((size_t)2 * kVPairs * kVPairLd + (size_t)warps * 4 * kBJ * nbp);
+}
+__global__ void __launch_bounds__(32 * kVMaxWarps)
+jacobi_v_kernel(float *__restrict__ V, const float *__restrict__ J, int n, int nbp,
+                const unsigned *__restrict__ state) {
+    extern __shared__ __align__(16) float vsm[];
+    const unsigned done = state[1];
+    if (done == 0)
+        return; // no sweep yet: V = I
+    const int s = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rounds = nbp - 1, pairs = nbp / 2, chunks = (pairs + kVPairs - 1) / kVPairs;
+    const int nb = (n + kBJ - 1) / kBJ, total = rounds * chunks;
+    const float *Jg = J + ((size_t)((done - 1) & 1) * gridDim.y + s) * rounds * pairs * kBJFloats;
+    // chunk c of the sweep: pairs p0 .. of one round, into buffer c & 1
+    auto stage = [&](int c) {
+        const int round = c / chunks, p0 = (c - round * chunks) * kVPairs;
+        const int count = min(kVPairs, pairs - p0);
+        const float *src = Jg + ((size_t)round * pairs + p0) * kBJFloats;
+        float *dst = vsm + (c & 1) * kVPairs * kVPairLd;
+        for (int e = threadIdx.x; e < count * (kBJFloats / 4); e += blockDim.x) {
+            const int p = e / (kBJFloats / 4), q = e - p * (kBJFloats / 4);
+            cp_async16(dst + p * kVPairLd + 4 * q, src + 4 * (size_t)e, 16);
+        }
+        cp_async_commit();
+    };
+    stage(0);
+    float4 *vr = reinterpret_cast<float4 *>(vsm + 2 * kVPairs * kVPairLd) + (size_t)warp * kBJ * nbp;
+    const int row = (blockIdx.x * (blockDim.x >> 5) + warp) * 4;
+    float *Vg = V + (size_t)s * n * n;
+    for (int c = lane; c < kBJ * nbp; c += 32) {
+        const float *g = Vg + (size_t)c * n + row;
+        vr[c] = make_float4(c < n && row < n ? g[0] : 0.f, c < n && row + 1 < n ? g[1] : 0.f,
+                            c < n && row + 2 < n ? g[2] : 0.f, c < n && row + 3 < n ? g[3] : 0.f);
+    }
+    for (int c = 0; c < total; c++) {
+        cp_async_wait<0>();
+        __syncthreads(); // chunk c is in place, chunk c - 1 is read
+        if (c + 1 < total)
+            stage(c + 1);
+        const int round = c / chunks, p0 = (c - round * chunks) * kVPairs;
+        const float *Jc = vsm + (c & 1) * kVPairs * kVPairLd;
+        float4 acc[kVTiles][4]; // by column
+        int first[kVTiles];     // the tile's first column, -1: none
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+        for (int u = 0; u < kVTiles; u++) {
+            const int tile = lane + 32 * u, p = tile / (kBCols / 4), cg = 4 * (tile % (kBCols / 4));
+            int bp, bq;
+            round_robin(nbp, round, min(p0 + p, pairs - 1), bp, bq);
+            // the bye (a sweep's first round also rotates within its block)
+            const bool on = p0 + p < pairs && (bq < nb || round == 0);
+            first[u] = !on ? -1 : cg < kBJ ? bp * kBJ + cg : bq * kBJ + cg - kBJ;
+            if (!on)
+                continue;
+            const float4 *vp = vr + bp * kBJ, *vq = vr + bq * kBJ - kBJ;
+            const float *j = Jc + p * kVPairLd + cg;
 #pragma unroll
             for (int v = 0; v < 4; v++)
-                acc[u][v] = 0.f;
-#pragma unroll 8
-        for (int i = 0; i < kBCols; i++) {
-            const float4 vin = *reinterpret_cast<const float4 *>(vb + (size_t)i * ld + rg);
-            const float4 jr = *reinterpret_cast<const float4 *>(&Jr[i][cg]);
-            const float vi[4] = {vin.x, vin.y, vin.z, vin.w}, ji[4] = {jr.x, jr.y, jr.z, jr.w};
+                acc[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < 4; u++)
+            for (int i = 0; i < kBCols; i++) {
+                const float4 x = i < kBJ ? vp[i] : vq[i];
+                const float4 jr = *reinterpret_cast<const float4 *>(j + i * kBCols);
+                const float jv[4] = {jr.x, jr.y, jr.z, jr.w};
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    acc[u][v].x = fmaf(x.x, jv[v], acc[u][v].x);
+                    acc[u][v].y = fmaf(x.y, jv[v], acc[u][v].y);
+                    acc[u][v].z = fmaf(x.z, jv[v], acc[u][v].z);
+                    acc[u][v].w = fmaf(x.w, jv[v], acc[u][v].w);
+                }
+            }
+        }
+        __syncwarp(); // the rows are read
+#pragma unroll
+        for (int u = 0; u < kVTiles; u++)
+            if (first[u] >= 0)
 #pragma unroll
                 for (int v = 0; v < 4; v++)
-                    acc[u][v] = fmaf(vi[u], ji[v], acc[u][v]);
-        }
-    };
-    auto put_tile = [&](float *vb, int ld, const float (&acc)[4][4]) {
+                    vr[first[u] + v] = acc[u][v];
+        __syncwarp();
+    }
+    for (int c = lane; c < n; c += 32) {
+        float *g = Vg + (size_t)c * n + row;
+        const float4 x = vr[c];
+        const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int v = 0; v < 4; v++)
-            *reinterpret_cast<float4 *>(vb + (size_t)(cg + v) * ld + rg) =
-                make_float4(acc[0][v], acc[1][v], acc[2][v], acc[3][v]);
-    };
-    if constexpr (kWholeV) {
-        constexpr int kPasses = (NP + kVRows - 1) / kVRows; // 1 or 2
-        cp_async_wait<0>();
-        __syncthreads(); // V block and Jr in place
-        float acc[kPasses][4][4];
-#pragma unroll
-        for (int ps = 0; ps < kPasses; ps++)
-            if (ps * kVRows + rg < NP)
-                vj_tile(Vb + ps * kVRows, VLD, acc[ps]);
-        __syncthreads(); // every thread has read Vb
-#pragma unroll
-        for (int ps = 0; ps < kPasses; ps++)
-            if (ps * kVRows + rg < NP)
-                put_tile(Vb + ps * kVRows, VLD, acc[ps]);
-        __syncthreads();
-        store_cols(Vg, Vb, VLD, n, 0, NP, gcol);
-    } else {
-        for (int r0 = 0; r0 < n; r0 += kVRows) {
-            if (r0 > 0) {
-                __syncthreads(); // the previous chunk is written out
-                stage_cols_async(Vb, VLD, Vg, n, r0, kVRows, gcol);
-                cp_async_commit();
-            }
-            cp_async_wait<0>();
-            __syncthreads(); // chunk and Jr in place
-            float acc[4][4];
-            vj_tile(Vb, VLD, acc);
-            __syncthreads(); // every thread has read the chunk
-            put_tile(Vb, VLD, acc);
-            __syncthreads();
-            store_cols(Vg, Vb, VLD, n, r0, kVRows, gcol);
-        }
+            if (row + v < n)
+                g[v] = xv[v];
     }
 }
 
@@ -1773,9 +1809,14 @@ cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino,
     return cudaGetLastError();
 }
 
+static int nos_blocks(int n) { // of kBJ columns, an even number
+    const int nb = (n + kBJ - 1) / kBJ;
+    return nb + (nb & 1);
+}
+
 template <int K4>
 static cudaError_t block_rounds(int n, int n_sino, const NosWork &w, cudaStream_t st) {
-    const int nb = (n + kBJ - 1) / kBJ, nbp = nb + (nb & 1);
+    const int nbp = nos_blocks(n);
     const size_t smem = sizeof(float) * block_round_smem_floats(K4);
     if (128 * K4 < n)
         return cudaErrorInvalidValue;
@@ -1783,13 +1824,45 @@ static cudaError_t block_rounds(int n, int n_sino, const NosWork &w, cudaStream_
         return cudaErrorInvalidValue;
     for (int r = 0; r < nbp - 1; r++)
         rt_block_round_kernel<K4><<<dim3(nbp / 2, n_sino), kBThreads, smem, st>>>(
-            w.X, w.V, n, nbp, r, w.off_bits, w.tiny);
+            w.X, w.J, n, nbp, r, w.off_bits, w.tiny, w.sweep_state);
+    return cudaGetLastError();
+}
+
+size_t nos_rotation_floats(int n, int n_sino) {
+    const size_t nbp = nos_blocks(n);
+    return 2 * n_sino * (nbp - 1) * (nbp / 2) * kBJFloats;
+}
+
+// Eight warps per CTA where the sweeps' rounds fill the machine (fewer copies of the
+// J's: 76.5 against 78.3 ms at 8 x 5795 x 720), else four (7.78 against 7.90 at
+// 8 x 1449 x 360).
+static cudaError_t rotate_v(int n, int n_sino, const NosWork &w, cudaStream_t st) {
+    const int nbp = nos_blocks(n);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int warps = nbp / 2 * n_sino > sms ? kVMaxWarps : 4, rows = 4 * warps;
+    const size_t smem = jacobi_v_smem(nbp, warps); // 209 KB at 1024 columns and 8 warps
+    if (smem > opt_in_smem((const void *)jacobi_v_kernel))
+        return cudaErrorInvalidValue;
+    jacobi_v_kernel<<<dim3((n + rows - 1) / rows, n_sino), 32 * warps, smem, st>>>(
+        w.V, w.J, n, nbp, w.sweep_state);
     return cudaGetLastError();
 }
 
 cudaError_t launch_nos_sweep(int n, int n_sino, const NosWork &w, int max_sweeps,
-                             cudaGraphConditionalHandle loop, cudaStream_t st) {
+                             cudaGraphConditionalHandle loop, cudaStream_t st, cudaStream_t side,
+                             cudaEvent_t fork, cudaEvent_t join) {
     cudaError_t e = cudaMemsetAsync(w.off_bits, 0, sizeof(unsigned) * n_sino, st);
+    // the previous sweep's rotations of V beside this sweep's rounds
+    if (e == cudaSuccess)
+        e = cudaEventRecord(fork, st);
+    if (e == cudaSuccess)
+        e = cudaStreamWaitEvent(side, fork, 0);
+    if (e == cudaSuccess)
+        e = rotate_v(n, n_sino, w, side);
+    if (e == cudaSuccess)
+        e = cudaEventRecord(join, side);
     if (e != cudaSuccess)
         return e;
     if (n <= 128)
@@ -1806,6 +1879,9 @@ cudaError_t launch_nos_sweep(int n, int n_sino, const NosWork &w, int max_sweeps
         e = block_rounds<8>(n, n_sino, w, st);
     else
         e = cudaErrorInvalidValue; // more than 1024 angles
+    if (e != cudaSuccess)
+        return e;
+    e = cudaStreamWaitEvent(st, join, 0);
     if (e != cudaSuccess)
         return e;
     nos_sweep_check_kernel<<<1, 32, 0, st>>>(w.off_bits, n_sino, w.sweep_state, max_sweeps,
@@ -1857,6 +1933,9 @@ cudaError_t launch_nos_assemble(const float2 *A, const NosDesc *desc, int n, int
                                 int max_m, const NosWork &w, float *out, cudaStream_t st) {
     const long long nn = (long long)n * n;
     const dim3 ge((unsigned)((nn + 255) / 256), n_sino), gt((n + kGemmTile - 1) / kGemmTile, (n + kGemmTile - 1) / kGemmTile, n_sino);
+    const cudaError_t e = rotate_v(n, n_sino, w, st); // the last sweep's
+    if (e != cudaSuccess)
+        return e;
     rt_invnorm_kernel<<<dim3((n + 3) / 4, n_sino), 128, 0, st>>>(w.X, n, w.tiny, w.inv);
     rt_scale_kernel<<<ge, 256, 0, st>>>(w.X, w.inv, n);
     // P = V U^T, then one Newton-Schulz step P <- P (3 I - P^T P) / 2 (in the
