@@ -828,7 +828,11 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
         a_elems += (size_t)d.ld * cols;
         out_elems += (size_t)d.m * cols;
     }
-    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * a_elems));
+    // the captured graphs hold these buffers' addresses, so they are sized for the
+    // longest columns of the row class: other images of a size then find
+    // them, and the graphs, as they are
+    const int class_m = tt::nos_class_rows(max_m);
+    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, (size_t)class_m * ncol)));
     TT_CHECK(p->ensure(p->nos_desc, sizeof(NosDesc) * n_sino));
     TT_CHECK(p->ensure(p->nos, sizeof(float) * out_elems));
     if (max_m > tt::nos_max_rows())
@@ -846,9 +850,9 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
                         sizeof(float) * n_sino + sizeof(unsigned) * 2;
     const size_t wy_at = (head + 255) & ~size_t(255);
     const size_t rotations = tt::nos_rotation_floats(cols, n_sino); // a multiple of 64
-    TT_CHECK(p->ensure(p->nos_work,
-                       wy_at + sizeof(float) * (rotations +
-                                                tt::nos_assemble_floats(cols, n_sino, max_m))));
+    const size_t assemble = std::max(tt::nos_assemble_floats(cols, n_sino, max_m),
+                                     tt::nos_assemble_floats(cols, n_sino, class_m));
+    TT_CHECK(p->ensure(p->nos_work, wy_at + sizeof(float) * (rotations + assemble)));
     tt::NosWork w;
     {
         char *q = (char *)p->nos_work.p;

@@ -238,6 +238,7 @@ int nos_ld(int m, int max_m);
 // QR serves one class).
 constexpr int kNosQrClasses = 7;
 int nos_qr_class(int max_m);
+int nos_class_rows(int max_m); // longest column of max_m's class
 // One Jacobi sweep on X (n - 1 + (n & 1) launches), then the stop rule on
 // the device: the sweep sets the while-loop condition `loop` to 0 when the
 // iteration has converged or max_sweeps sweeps are done (w.sweep_state,

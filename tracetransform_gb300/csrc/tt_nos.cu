@@ -1769,6 +1769,11 @@ int nos_qr_class(int max_m) {
     return c;
 }
 
+int nos_class_rows(int max_m) {
+    const QrClass c = kQrClasses[nos_qr_class(max_m)];
+    return std::max(max_m, 2 * c.threads * c.pairs);
+}
+
 int nos_ld(int m, int max_m) {
     const int rows = 2 * kQrClasses[nos_qr_class(max_m)].threads;
     return (m + rows - 1) / rows * rows;
