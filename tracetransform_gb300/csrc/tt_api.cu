@@ -832,7 +832,8 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     // longest columns of the row class: other images of a size then find
     // them, and the graphs, as they are
     const int class_m = tt::nos_class_rows(max_m);
-    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, (size_t)class_m * ncol)));
+    const size_t class_elems = (size_t)tt::nos_ld(class_m, class_m) * ncol;
+    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, class_elems)));
     TT_CHECK(p->ensure(p->nos_desc, sizeof(NosDesc) * n_sino));
     TT_CHECK(p->ensure(p->nos, sizeof(float) * out_elems));
     if (max_m > tt::nos_max_rows())

@@ -231,8 +231,8 @@ cudaError_t launch_nos_align(const float *sino, int rows, int cols, int n_sino,
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
                               const NosWork &w, cudaStream_t st);
 int nos_max_rows(); // aligned rows the QR kernels hold in registers
-// Leading dimension of an aligned matrix of m rows, max_m the call's largest: whole
-// pairs of rows for every thread of the QR's CTAs.
+// Leading dimension of an aligned matrix of m rows, max_m the call's largest: the rows
+// and as many zeros as the QR's CTAs have threads.
 int nos_ld(int m, int max_m);
 // Which of its kernels the QR takes for columns of up to max_m rows (a captured
 // QR serves one class).

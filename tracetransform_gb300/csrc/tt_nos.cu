@@ -323,40 +323,41 @@ template <int GB> __device__ __forceinline__ float2 qr_warp_sums(float2 (&v)[GB]
 // the stored column that ends at position k.
 //
 // What bounds a step is the instructions issued per element, then the chain
-// map, pivot, pivot column, sums, scalars, update.  So thread t holds the row
-// pairs 2 (t + T u), u0 <= u < nu, whatever k is, in columns padded with
-// zeros to whole slots: every access is 16 bytes at a constant offset from one
-// pointer per column, and no row is tested -- x is zero up to row k, which leaves
-// the rows above untouched.  A group's columns come in by asynchronous copies
-// issued before the pivot is known, into slots of shared memory that only
-// their own thread reads (no barrier); a slot is refilled for the next group
-// once its column is written.  The sums of a whole group and |x|^2 share one
-// barrier, lane g of every warp then forms column g's scalars, and the two
-// divisions of the reflector run in two lanes.  Sums, updates and scalars
-// are all double-float.
-// The whole orthonormal circus, before (8-byte accesses, each with its own address
-// and row test, a reduction and a barrier per column) and now: 8 x 1449 x 360,
-// 9.28 and 8.3 ms; 4 x 450 x 360, 6.16 and 5.7; 8 x 5795 x 720, 90.6 and 78.8.  Two
-// rows at a time in packed operations take 40 % fewer instructions and as
-// long: a step then waits for its chain.
+// map, pivot, pivot column, sums, scalars, update.  Thread t holds rows
+// k + 1 + t + T u, u < keff, of columns padded with zeros (nos_ld): every access is at a
+// constant offset from one pointer per column, and no row is tested.  A
+// group's columns come in by asynchronous copies issued before the pivot is
+// known, into slots of shared memory that only their own thread reads (no
+// barrier); a slot is refilled for the next group once its column is written.
+// The sums of a whole group and |x|^2 share one barrier, lane g of every warp
+// then forms column g's scalars, and the two divisions of the reflector run in
+// two lanes.  Sums, updates and scalars are all double-float; their order
+// hangs on T alone (polar factors of nearly dependent columns change visibly
+// with their last bits).
+// The whole orthonormal circus, before (an address and a row test per access, a
+// reduction and a barrier per column) and after this alone: 8 x 1449 x 360, 9.28 and
+// 8.4; 4 x 450 x 360, 6.16 and 5.6; 8 x 5795 x 720, 90.6 and 87.  Two rows at a time in packed
+// operations took 40 % fewer instructions and as long: a step then waits for its
+// chain.
 //
-// K: row pairs per thread (2 K T >= ld).  CTAs per SM: by registers (four floats
-// per row pair of x, no spills) and by the slots' shared memory.  Groups of
-// two: of four, 8 x 1449 x 360 takes 8.45 against 8.31 ms in all (fewer CTAs fit);
-// of one, 8 x 5795 x 720 takes 86.9 against 78.8.
+// K: rows per thread.  CTAs per SM: by registers (two floats per row of x, and
+// more to have the column's loads in flight: bounds of 5 and 3 CTAs for K = 16 took
+// 10.7 ms at 8 x 1700 x 360 and 12.7 at 8 x 3000 x 360, these 9.6 and 11.0) and by the
+// slots' shared memory.  Groups of two: of four, fewer CTAs fit; of one, 8 x 5795
+// x 720 takes a tenth longer.
 constexpr int kQrGroup = 2;
 __host__ __device__ constexpr size_t qr_smem(int K, int T) {
-    return sizeof(float4) * (size_t)kQrGroup * K * T;
+    return sizeof(float2) * (size_t)kQrGroup * K * T;
 }
 __host__ __device__ constexpr int qr_ctas(int K, int T) {
-    return T == 64 ? 10 : T == 128 ? (K == 4 ? 6 : 5) : K == 8 ? 3 : K == 12 ? 2 : 1;
+    return T == 128 ? (K == 4 ? 8 : K == 8 ? 6 : 3) : 1;
 }
 template <int K, int T>
 __global__ void __launch_bounds__(T, qr_ctas(K, T))
 qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, int n_sino,
                int k, NosWork w) {
     constexpr int kW = T / 32, GB = kQrGroup, kStep = 32 / GB;
-    extern __shared__ __align__(16) float4 s_slot[]; // [GB][K][T]
+    extern __shared__ __align__(16) float2 s_slot[]; // [GB][K][T]
     __shared__ int s_bv[kW];
     __shared__ int s_bi[kW];
     __shared__ float2 s_xn[kW];
@@ -366,8 +367,7 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const NosDesc d = desc[s];
     const size_t ld = d.ld;
-    // the first slot with rows below k and the slots in all
-    const int u0 = (k + 1) / (2 * T), nu = d.ld / (2 * T);
+    const int keff = (d.m - k - 1 + T - 1) / T; // slots that cover the rows below k
     float2 *As = A + d.a_off;
     const size_t cur = (size_t)(k & 1) * n_sino + s, nxt = (size_t)((k + 1) & 1) * n_sino + s;
     const float2 *nr = w.norms + cur * n;
@@ -375,18 +375,18 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
     float *og = w.orig + (size_t)s * n;
     const int j0 = k + b, cnt = (n - j0 + G - 1) / G;
     const int g_mine = lane % GB;   // the group's column whose scalars this lane forms
-    float4 *slot = s_slot + threadIdx.x;
-    auto column = [&](int c) { // this thread's row pairs of column c, T apart
-        return reinterpret_cast<float4 *>(As + c * ld) + threadIdx.x;
+    float2 *slot = s_slot + threadIdx.x;
+    auto below = [&](int c) { // this thread's rows of column c, T apart
+        return As + c * ld + k + 1 + threadIdx.x;
     };
     auto issue = [&](int g, int c) { // column c into the slots of group member g
-        const float4 *src = column(c);
+        const float2 *src = below(c);
         const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + g * K * T);
 #pragma unroll
         for (int u = 0; u < K; u++)
-            if (u >= u0 && u < nu)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 dst + (unsigned)(u * T * sizeof(float4))),
+            if (u < keff)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                 dst + (unsigned)(u * T * sizeof(float2))),
                              "l"(src + u * T)
                              : "memory");
     };
@@ -444,31 +444,18 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
             bidx = s_bi[u];
         }
     const int p = bidx >> 16, cp = bidx & 0xffff;
-    const float4 *x = column(cp);
-    float4 xv[K];
+    const float2 *x = below(cp);
+    float2 xv[K];
 #pragma unroll
     for (int u = 0; u < K; u++)
-        xv[u] = u >= u0 && u < nu ? x[u * T] : make_float4(0.f, 0.f, 0.f, 0.f);
+        xv[u] = u < keff ? x[u * T] : make_float2(0.f, 0.f);
     const float2 xk = As[cp * ld + k];
-    const int head = k - 2 * (int)(threadIdx.x + T * u0); // zero rows <= k of slot u0
-    if (head >= 0)
-#pragma unroll
-        for (int u = 0; u < K; u++)
-            if (u == u0) {
-                xv[u].x = xv[u].y = 0.f;
-                if (head >= 1)
-                    xv[u].z = xv[u].w = 0.f;
-            }
-    auto dot = [](DfDot (&acc)[2], float4 a, float4 c) {
-        df_dot_add(acc[0], make_float2(a.x, a.y), make_float2(c.x, c.y));
-        df_dot_add(acc[1], make_float2(a.z, a.w), make_float2(c.z, c.w));
-    };
     {
         DfDot dn[2];
 #pragma unroll
         for (int u = 0; u < K; u++)
-            if (u >= u0 && u < nu)
-                dot(dn, xv[u], xv[u]);
+            if (u < keff)
+                df_dot_add(dn[u & 1], xv[u], xv[u]);
         float2 xn = df_add(df_dot_end(dn[0]), df_dot_end(dn[1]));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -490,8 +477,8 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
             if (g < live) // uniform
 #pragma unroll
                 for (int u = 0; u < K; u++)
-                    if (u >= u0 && u < nu)
-                        dot(dv, xv[u], slot[(g * K + u) * T]);
+                    if (u < keff)
+                        df_dot_add(dv[u & 1], xv[u], slot[(g * K + u) * T]);
             v[g] = df_add(df_dot_end(dv[0]), df_dot_end(dv[1]));
         }
         const float2 part = qr_warp_sums<GB>(v, lane);
@@ -548,14 +535,6 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
         const bool rec = on && n2.x <= 1.5e-8f * o_mine;
         const unsigned rec_mask = __ballot_sync(TT_FULL_MASK, rec);
         const unsigned on_mask = __ballot_sync(TT_FULL_MASK, on);
-        // a[k] into its slot, if that is among the rewritten ones (u0 may be past it)
-        const int pair_k = (k >> 1) - T * u0;
-        const bool k_inside = pair_k >= 0;
-        if (k_inside && pair_k >> 5 == warp) {
-            if (lane < GB && on)
-                reinterpret_cast<float2 *>(s_slot + (g_mine * K + u0) * T + pair_k)[k & 1] = k_mine;
-            __syncwarp();
-        }
         const int c_now = c_mine;
         const float2 k_now = k_mine;
         if (t0 + GB < cnt) { // the next group's column of this lane
@@ -575,32 +554,20 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
             if (on_mask >> g & 1) { // uniform
                 const bool again = rec_mask >> g & 1;
                 if (!zero) {
-                    float4 *c = column(cj);
+                    float2 *c = below(cj);
 #pragma unroll
                     for (int u = 0; u < K; u++)
-                        if (u >= u0 && u < nu) {
-                            const float4 a = slot[(g * K + u) * T], xu = xv[u];
-                            const float2 lo = df_fma(f, make_float2(xu.x, xu.y),
-                                                     make_float2(a.x, a.y));
-                            const float2 hi = df_fma(f, make_float2(xu.z, xu.w),
-                                                     make_float2(a.z, a.w));
-                            c[u * T] = make_float4(lo.x, lo.y, hi.x, hi.y);
-                        }
+                        if (u < keff)
+                            c[u * T] = df_fma(f, xv[u], slot[(g * K + u) * T]);
                 }
                 if (again) { // rare: the norm of the new column below row k
                     DfDot dr[2];
-                    for (int u = u0; u < nu; u++) {
-                        float4 a = slot[(g * K + u) * T];
-                        const float4 *c = column(cj);
-                        if (!zero)
-                            a = c[u * T]; // as this thread wrote it
-                        const int row = 2 * (threadIdx.x + T * u);
-                        if (row <= k)
-                            a.x = a.y = 0.f;
-                        if (row + 1 <= k)
-                            a.z = a.w = 0.f;
-                        dot(dr, a, a);
-                    }
+#pragma unroll
+                    for (int u = 0; u < K; u++)
+                        if (u < keff) { // as this thread wrote it
+                            const float2 a = zero ? slot[(g * K + u) * T] : below(cj)[u * T];
+                            df_dot_add(dr[u & 1], a, a);
+                        }
                     const float2 r = qr_block_sum<T>(
                         df_add(df_dot_end(dr[0]), df_dot_end(dr[1])), s_red[rb]);
                     rb ^= 1;
@@ -617,7 +584,7 @@ qr_step_kernel(float2 *__restrict__ A, const NosDesc *__restrict__ desc, int n, 
             }
         }
         if (on && threadIdx.x < GB) {
-            if (!zero && !k_inside)
+            if (!zero)
                 As[c_now * ld + k] = k_now;
             const int dest = j == k ? p : j;
             w.norms[nxt * n + dest] = n2;
@@ -1753,31 +1720,30 @@ static cudaError_t qr_steps(float2 *A, const NosDesc *desc, int n, int n_sino, c
 
 int nos_max_rows() { return 32 * kQrThreads; }
 
-// Threads per CTA and row pairs per thread of the QR by longest column: a warp
-// has about a thousand instructions a step to do whatever its columns' length,
-// so short columns take fewer warps.
+// Threads per CTA and rows per thread of the QR by longest column: 128 threads up to
+// 2048 rows (more CTAs, and so more column chains, in flight per SM), 256
+// above; short columns take fewer rows per thread, so fewer registers and more
+// CTAs per SM with fewer columns each.
 struct QrClass {
-    int threads, pairs;
+    int threads, rows;
 };
-constexpr QrClass kQrClasses[kNosQrClasses] = {{64, 4},  {128, 4},  {128, 6}, {128, 8},
-                                               {256, 8}, {256, 12}, {256, 16}};
+constexpr QrClass kQrClasses[kNosQrClasses] = {{128, 4},  {128, 8},  {128, 12}, {128, 16},
+                                               {256, 16}, {256, 24}, {256, 32}};
 
 int nos_qr_class(int max_m) {
     int c = 0;
-    while (c < kNosQrClasses - 1 && max_m > 2 * kQrClasses[c].threads * kQrClasses[c].pairs)
+    while (c < kNosQrClasses - 1 && max_m > kQrClasses[c].threads * kQrClasses[c].rows)
         c++;
     return c;
 }
 
 int nos_class_rows(int max_m) {
     const QrClass c = kQrClasses[nos_qr_class(max_m)];
-    return std::max(max_m, 2 * c.threads * c.pairs);
+    return std::max(max_m, c.threads * c.rows);
 }
 
-int nos_ld(int m, int max_m) {
-    const int rows = 2 * kQrClasses[nos_qr_class(max_m)].threads;
-    return (m + rows - 1) / rows * rows;
-}
+// A column step reads and writes up to threads - 1 rows past the last.
+int nos_ld(int m, int max_m) { return (m + kQrClasses[nos_qr_class(max_m)].threads + 3) & ~3; }
 
 cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino, int max_m,
                               const NosWork &w, cudaStream_t st) {
@@ -1787,25 +1753,25 @@ cudaError_t launch_nos_factor(float2 *A, const NosDesc *desc, int n, int n_sino,
     cudaError_t e = cudaSuccess;
     switch (nos_qr_class(max_m)) {
     case 0:
-        e = qr_steps<kQrClasses[0].pairs, kQrClasses[0].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[0].rows, kQrClasses[0].threads>(A, desc, n, n_sino, w, st);
         break;
     case 1:
-        e = qr_steps<kQrClasses[1].pairs, kQrClasses[1].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[1].rows, kQrClasses[1].threads>(A, desc, n, n_sino, w, st);
         break;
     case 2:
-        e = qr_steps<kQrClasses[2].pairs, kQrClasses[2].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[2].rows, kQrClasses[2].threads>(A, desc, n, n_sino, w, st);
         break;
     case 3:
-        e = qr_steps<kQrClasses[3].pairs, kQrClasses[3].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[3].rows, kQrClasses[3].threads>(A, desc, n, n_sino, w, st);
         break;
     case 4:
-        e = qr_steps<kQrClasses[4].pairs, kQrClasses[4].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[4].rows, kQrClasses[4].threads>(A, desc, n, n_sino, w, st);
         break;
     case 5:
-        e = qr_steps<kQrClasses[5].pairs, kQrClasses[5].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[5].rows, kQrClasses[5].threads>(A, desc, n, n_sino, w, st);
         break;
     default:
-        e = qr_steps<kQrClasses[6].pairs, kQrClasses[6].threads>(A, desc, n, n_sino, w, st);
+        e = qr_steps<kQrClasses[6].rows, kQrClasses[6].threads>(A, desc, n, n_sino, w, st);
     }
     if (e != cudaSuccess)
         return e;
