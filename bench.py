@@ -774,13 +774,13 @@ def run_single(args, world, rank, local_rank):
     ms = max_over_ranks(ms, world)
     # sinograms, circus, z-score; with the Hermite circus: weighted-median
     # offsets, alignment, QR (qr_init, one launch per column step, R^T), the
-    # sweeps (one launch per block round), assembly (6), one circus launch
-    # per sinogram and a z-score
+    # sweeps (one launch per block round, V's rotations, the stop rule),
+    # assembly (8), one circus launch per sinogram and a z-score
     launches = 3
     if herm:
-        nb = (A + 15) // 16  # 16-column blocks, nbp - 1 block rounds per sweep
+        nb = (A + 11) // 12  # 12-column blocks, nbp - 1 block rounds per sweep
         nbp = nb + (nb & 1)
-        launches += 2 + (A + 2) + eng.last_sweeps * (nbp - 1) + 6 + len(tfs) + 1
+        launches += 2 + (A + 2) + eng.last_sweeps * (nbp + 1) + 8 + len(tfs) + 1
 
     # end to end: one C ABI call with host buffers (pinned)
     h_img = torch.from_numpy(np.ascontiguousarray(img.ravel(order="F"))).pin_memory()

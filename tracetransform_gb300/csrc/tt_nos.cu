@@ -10,7 +10,7 @@
 // dominate), double-float pairs on the FP32 pipes where float is too short:
 //
 //   nos_offsets   per column: weighted median row - center, with the
-//                 reference's sequential float sums (one thread per column)
+//                 reference's sequential float sums (one warp per column)
 //   nos_align     the shifted columns into a zeroed m x A matrix of
 //                 double-float pairs (hi + lo, ~48 significant bits)
 //   QR            column-pivoting Householder QR, A P = Q R, in double-float
