@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 import tracetransform_gb300 as tt
+from tracetransform_gb300._native import TTError
 
 pytestmark = pytest.mark.gpu
 
@@ -26,3 +27,18 @@ def test_alignment_medians(rows):
     got, c = tt.nearest_orthonormal_sinogram(np.asfortranarray(sino))
     assert got.shape == (rows + abs(mx) + abs(mn), cols)
     assert c == center + mx
+
+
+@pytest.mark.parametrize("rows", [8190, 8191, 8193, 9001])
+def test_longest_columns(rows):
+    """Up to 8192 aligned rows are taken; more are refused with their number,
+    whichever kernel finds the medians."""
+    rng = np.random.default_rng(rows)
+    sino = (0.05 * rng.random((rows, 3))).astype(np.float32)
+    sino[(rows - 1) // 2 + 1] += rows  # every median one row past the center: |1| + |1| rows more
+    if rows + 2 <= 8192:
+        got, c = tt.nearest_orthonormal_sinogram(np.asfortranarray(sino))
+        assert got.shape == (rows + 2, 3) and c == (rows - 1) // 2 + 1
+    else:
+        with pytest.raises(TTError, match=f"{rows + 2} aligned rows exceeds 8192"):
+            tt.nearest_orthonormal_sinogram(np.asfortranarray(sino))
