@@ -200,17 +200,24 @@ __device__ __forceinline__ void fft_convolve(float2 *s, const float2 *__restrict
     fft_convolve_from<LOGM, LOGM, fft_lead(LOGM)>(s, tw, filt, load);
 }
 
-// 2^-e and 2^e for a column of squared norm ss, e half of its exponent, so
-// that both columns of a pair enter the transform with norms of about one
-// (a small column must not drown in the rounding of a large neighbour).
+// Whether two columns of squared norms q1 and q2 share a transform: both are
+// normal floats.  A zero, subnormal or non-finite one has no scale below that
+// brings its column to its neighbour's size; such columns take transforms of
+// their own, as they are.
+__device__ __forceinline__ bool pair_shares(float q1, float q2) {
+    const float inf = __int_as_float(0x7f800000);
+    return q1 >= 0x1p-126f && q2 >= 0x1p-126f && q1 < inf && q2 < inf;
+}
+
+// 2^-e and 2^e for a column of squared norm ss (a normal float, else of no
+// use), e half of its exponent, so that both columns of a pair enter the
+// transform with norms of about one (a small column must not drown in the
+// rounding of a large neighbour).
 struct PairScale {
     float down, up;
 };
 __device__ __forceinline__ PairScale pair_scale(float ss) {
-    const int e2 = ((__float_as_int(ss) >> 23) & 0xff) - 127;
-    if (!(ss > 0.f) || e2 < -126 || e2 > 127) // zero, subnormal, not finite: as they are
-        return PairScale{1.f, 1.f};
-    const int e = e2 >> 1; // within -63 .. 63
+    const int e = (((__float_as_int(ss) >> 23) & 0xff) - 127) >> 1; // -63 .. 63 if normal
     return PairScale{__int_as_float((127 - e) << 23), __int_as_float((127 + e) << 23)};
 }
 
