@@ -155,7 +155,11 @@ struct tt_plan {
     std::map<int, float2 *> t345;                       // n -> 3 x n
     std::map<int, FftTables> fft;                       // n -> P3 tables
     std::map<std::tuple<int, int, int>, float *> herm;  // (n, order, center)
-    std::map<std::vector<float>, float2 *> trig;        // angle list -> (c, s)
+    struct Trig {
+        float2 *cs;  // (c, s) of every angle
+        bool finite; // of all of them
+    };
+    std::map<std::vector<float>, Trig> trig;            // angle list -> its table
     std::map<std::vector<long>, const float **> herm_ptrs;
     DevBuf in, stretch, sino, circ, sig, region, nos, batch_in, batch_out, params;
     // P-stage scratch: P3 partial sums, the exact-sort list of P2 (count + entries)
@@ -414,21 +418,23 @@ struct tt_plan {
         return TT_OK;
     }
 
-    tt_status get_trig(const float *angles, int n_angles, const float2 **out) {
+    tt_status get_trig(const float *angles, int n_angles, const float2 **out,
+                       bool *finite = nullptr) {
         std::vector<float> key(angles, angles + n_angles);
         auto it = trig.find(key);
-        if (it != trig.end()) {
-            *out = it->second;
-            return TT_OK;
+        if (it == trig.end()) {
+            std::vector<float2> h(n_angles);
+            Trig t{nullptr, true};
+            for (int a = 0; a < n_angles; a++) {
+                h[a] = tt::rotation(angles[a]);
+                t.finite &= std::isfinite(h[a].x) && std::isfinite(h[a].y);
+            }
+            TT_CHECK(upload(&t.cs, h));
+            it = trig.emplace(key, t).first;
         }
-        std::vector<float2> h(n_angles);
-        for (int a = 0; a < n_angles; a++) {
-            h[a] = tt::rotation(angles[a]);
-        }
-        float2 *d;
-        TT_CHECK(upload(&d, h));
-        trig[key] = d;
-        *out = d;
+        *out = it->second.cs;
+        if (finite)
+            *finite = it->second.finite;
         return TT_OK;
     }
 
@@ -1280,9 +1286,10 @@ static tt_status sino_backward_impl(tt_plan *plan, int n_images, int src_rows, i
         !d_grad_sino || !d_medians || !d_grad_image)
         return fail(TT_ERR_INVALID_ARG, "bad geometry or buffers for the backward pass");
     const T *cs;
+    bool finite = false;
     if (sizeof(T) == sizeof(float)) {
         const float2 *t;
-        TT_CHECK(p->get_trig(angles_deg, n_angles, &t));
+        TT_CHECK(p->get_trig(angles_deg, n_angles, &t, &finite));
         cs = (const T *)t;
     } else {
         const double *t;
@@ -1295,7 +1302,7 @@ static tt_status sino_backward_impl(tt_plan *plan, int n_images, int src_rows, i
                        sizeof(T) * 4 * (size_t)n * std::max(n_angles, 1) * (size_t)n_images));
     TT_CUDA(tt::launch_sino_backward<T>(d_grad_sino, d_medians, n_images, n, n_angles, code, n_t,
                                         (T *)p->params.p, src_rows, src_cols, row_off, col_off,
-                                        cs, d_grad_image, pick_stream(p, stream)));
+                                        cs, finite, d_grad_image, pick_stream(p, stream)));
     return TT_OK;
 }
 } // extern "C++"

@@ -394,7 +394,8 @@ constexpr int kAdjWarps = 8; // angle groups per pixel group
 // each): nearest lattice points come from an add of 1.5 2^23 whose low bits are
 // the index (no conversions), a column's parameters from one address, the tent
 // weights from saturating adds.  64 images of 256^2 x 360 angles: 7.46 ms (8.94
-// with conversions, comparisons and per-angle index checks).
+// with conversions, comparisons and per-angle index checks).  Every (cos, sin)
+// has to be finite: nothing here tests the index.
 __device__ __forceinline__ float gather_inside(int n, int n_angles, int warp, float o, float dx,
                                                float dy, float fpx, float fpy,
                                                const float *__restrict__ cs,
@@ -461,7 +462,7 @@ __device__ __forceinline__ float gather_inside(int n, int n_angles, int warp, fl
 template <typename T, bool kInterior>
 __global__ void __launch_bounds__(32 * kAdjWarps)
 adjoint_gather_kernel(int rows, int cols, int row_off, int col_off, int n, int n_angles,
-                      const T *__restrict__ cs, const T *__restrict__ params,
+                      const T *__restrict__ cs, bool finite, const T *__restrict__ params,
                       T *__restrict__ grad_img) {
     using C = Coord<T>;
     __shared__ T part[kAdjWarps][32];
@@ -478,8 +479,9 @@ adjoint_gather_kernel(int rows, int cols, int row_off, int col_off, int n, int n
         const T dx = fpx - o, dy = fpy - o;
         // pixels further than two from the circle inside the frame keep their
         // 3 x 3 block inside the lattice at every angle (all but the frame's
-        // corners): no index checks
-        if (kInterior && sizeof(T) == sizeof(float) &&
+        // corners): no index checks.  Not with an angle that is no number: its
+        // lattice point is none either, and only the general form tests it.
+        if (kInterior && sizeof(T) == sizeof(float) && finite &&
             __all_sync(live, dx * dx + dy * dy <= (o - 2) * (o - 2))) {
             acc = gather_inside(n, n_angles, warp, (float)o, (float)dx, (float)dy, (float)fpx,
                                 (float)fpy, (const float *)cs, (const float *)params);
@@ -698,7 +700,7 @@ template <typename T>
 cudaError_t launch_sino_backward(const T *grad_sino, const int *medians, int n_images, int n,
                                  int n_angles, unsigned long long tf_code, int n_t, T *params,
                                  int rows, int cols, int row_off, int col_off, const T *cs,
-                                 T *grad_img, cudaStream_t st) {
+                                 bool finite, T *grad_img, cudaStream_t st) {
     if (n_images <= 0)
         return cudaSuccess;
     const long long lines = (long long)n * n_angles * n_images, pix = (long long)rows * cols;
@@ -709,10 +711,10 @@ cudaError_t launch_sino_backward(const T *grad_sino, const int *medians, int n_i
         const dim3 grid((unsigned)((pix + 31) / 32), n_images);
         if (interior_source(n, row_off, col_off, rows, cols))
             adjoint_gather_kernel<T, true><<<grid, 32 * kAdjWarps, 0, st>>>(
-                rows, cols, row_off, col_off, n, n_angles, cs, params, grad_img);
+                rows, cols, row_off, col_off, n, n_angles, cs, finite, params, grad_img);
         else
             adjoint_gather_kernel<T, false><<<grid, 32 * kAdjWarps, 0, st>>>(
-                rows, cols, row_off, col_off, n, n_angles, cs, params, grad_img);
+                rows, cols, row_off, col_off, n, n_angles, cs, finite, params, grad_img);
     }
     return cudaGetLastError();
 }
@@ -804,9 +806,10 @@ template cudaError_t launch_circus_backward<double>(const double *, int, int, in
                                                     cudaStream_t);
 template cudaError_t launch_sino_backward<float>(const float *, const int *, int, int, int,
                                                  unsigned long long, int, float *, int, int, int,
-                                                 int, const float *, float *, cudaStream_t);
+                                                 int, const float *, bool, float *, cudaStream_t);
 template cudaError_t launch_sino_backward<double>(const double *, const int *, int, int, int,
                                                   unsigned long long, int, double *, int, int, int,
-                                                  int, const double *, double *, cudaStream_t);
+                                                  int, const double *, bool, double *,
+                                                  cudaStream_t);
 
 } // namespace tt

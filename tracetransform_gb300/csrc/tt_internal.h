@@ -184,11 +184,12 @@ cudaError_t launch_circus_backward(const T *sino, int rows, int cols, int n_sino
 cudaError_t launch_circus_backward_fft(const float *sino, int rows, int cols, int n_sino,
                                        const int *d_kinds, int n_p, const float *grad_circus,
                                        const ChirpTables &t, int M, float *out, cudaStream_t st);
+// finite: every entry of cs is.
 template <typename T>
 cudaError_t launch_sino_backward(const T *grad_sino, const int *medians, int n_images, int n,
                                  int n_angles, unsigned long long tf_code, int n_t, T *params,
                                  int rows, int cols, int row_off, int col_off, const T *cs,
-                                 T *grad_img, cudaStream_t st);
+                                 bool finite, T *grad_img, cudaStream_t st);
 cudaError_t launch_sino_f64(const double *img, int rows, int cols, int row_off, int col_off,
                             int n, const double *cs, unsigned long long tf_code, int n_t,
                             int n_angles, double *out, int *medians, cudaStream_t st);
