@@ -45,3 +45,16 @@ def test_non_finite_angle_adds_nothing(bad, at):
 def test_all_angles_non_finite():
     eng = Engine(0)
     assert torch.all(_adjoint(eng, [np.nan, np.inf], _grad(2)) == 0)
+
+
+def test_a_list_with_nan_has_its_own_table():
+    """A NaN is neither below nor above any angle: a list holding one must not find
+    the table of a list that differs from it there, nor the other way round."""
+    angles, nan = [0, 17, 45], [0, np.nan, 45]
+    grad = _grad(3)
+    first, second = Engine(0), Engine(0)
+    want = _adjoint(first, angles, grad)
+    zeroed = _adjoint(first, nan, grad)
+    assert torch.equal(_adjoint(second, nan, grad), zeroed)
+    assert torch.equal(_adjoint(second, angles, grad), want)
+    assert not torch.equal(zeroed, want)

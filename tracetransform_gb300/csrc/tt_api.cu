@@ -159,7 +159,16 @@ struct tt_plan {
         float2 *cs;  // (c, s) of every angle
         bool finite; // of all of them
     };
-    std::map<std::vector<float>, Trig> trig;            // angle list -> its table
+    // Angle lists in the order of their bytes: a NaN compares as equal to every
+    // number, so by value a list that holds one would share another list's table.
+    struct BytesLess {
+        bool operator()(const std::vector<float> &a, const std::vector<float> &b) const {
+            if (a.size() != b.size())
+                return a.size() < b.size();
+            return !a.empty() && std::memcmp(a.data(), b.data(), sizeof(float) * a.size()) < 0;
+        }
+    };
+    std::map<std::vector<float>, Trig, BytesLess> trig; // angle list -> its table
     std::map<std::vector<long>, const float **> herm_ptrs;
     DevBuf in, stretch, sino, circ, sig, region, nos, batch_in, batch_out, params;
     // P-stage scratch: P3 partial sums, the exact-sort list of P2 (count + entries)
@@ -182,7 +191,7 @@ struct tt_plan {
     // backward / double-precision tables
     std::map<int, float *> dft32;                  // n -> cos, sin(2 pi j / n), 2 n
     std::map<int, double *> dft64, lin64;
-    std::map<std::vector<float>, double *> trig64; // angle list -> (cos, sin) in double
+    std::map<std::vector<float>, double *, BytesLess> trig64; // -> (cos, sin) in double
     std::map<std::vector<int>, int *> kinds;
 
     template <typename T> tt_status get_dft(int n, const T **cosv, const T **sinv) {
