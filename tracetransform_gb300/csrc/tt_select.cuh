@@ -8,13 +8,14 @@
 //   1. weights become u32 fixed point (2^-30 of a power-of-two bound on the
 //      total, so twice any sum fits 32 bits), summed exactly and
 //      deterministically by integer atomics;
-//   2. a 256-bin histogram linear in the key over [klo, khi] locates the bin
+//   2. a 256-bin histogram linear in the key over [0, top] locates the bin
 //      holding the crossing (bins are monotone in the key);
 //   3. the entries of that bin are collected, and each lane adds up the
 //      weights of the entries up to its own: the smallest that qualifies is
 //      the answer.  A bin of more than kSelList entries is refined first:
-//      its key range takes the histogram's place and step 2 repeats (a bin
-//      whose keys are all equal is the answer).
+//      step 2 repeats over its key range with bins linear in the keys' bit
+//      patterns, which no range is too narrow for (a bin whose keys are
+//      all equal is the answer).
 //
 // One warp per line.  What bounds it is the instruction count: a histogram
 // pass and a collecting pass over half the line, each with as little per
@@ -25,6 +26,8 @@
 // (3.21 with the bins recomputed by conversions and the weights in both
 // passes, 64-bit scans and a 64-entry bitonic sort).
 #pragma once
+
+#include <climits>
 
 #include "tt_common.cuh"
 
@@ -81,14 +84,19 @@ __device__ __forceinline__ float sel_scale(float total) {
     return __int_as_float((127 + 30 - E) << 23);
 }
 
-// Histogram bin of key k >= klo, bs = 256 / range: the integer that
-// (k - klo) bs rounds to, in the mantissa of 2^23, at most 255 -- monotone in
-// k.  A key below klo or NaN gives a valid bin too (255), so no input can
-// index outside the histogram; such keys carry no weight.
+// Bins per unit of a key in [0, top].  At most the largest float, which the
+// quotient exceeds for top < 2^-120: the bins are then wider than top / 256 but
+// still part the samples from the zeros.
+__device__ __forceinline__ float sel_per_key(float top) {
+    return fminf((float)kSelBins / top, 3.402823466e38f);
+}
+// Histogram bin of key k >= 0, bs = sel_per_key: the integer that k bs rounds
+// to, in the mantissa of 2^23, at most 255 -- monotone in k.  A negative or NaN
+// key gives a valid bin too (255), so no input can index outside the
+// histogram; such keys carry no weight.
 constexpr unsigned kSelOne = 0x4B000000u; // 2^23
-__device__ __forceinline__ unsigned sel_bin(float k, float klo, float bs) {
-    return min((unsigned)kSelBins - 1,
-               __float_as_uint(fmaf(k - klo, bs, 8388608.f)) - kSelOne);
+__device__ __forceinline__ unsigned sel_bin(float k, float bs) {
+    return min((unsigned)kSelBins - 1, __float_as_uint(fmaf(k, bs, 8388608.f)) - kSelOne);
 }
 
 __device__ __forceinline__ void sel_clear(SelScratch *sc, int lane) {
@@ -136,15 +144,15 @@ __device__ __forceinline__ SelPick sel_pick(const SelScratch *sc, unsigned below
     return p;
 }
 
-// Is key k in bin `bin` of a histogram from klo (bs as in sel_bin)?
+// Is key k in bin `bin` of a histogram (bs as in sel_bin)?
 struct SelTest {
-    float klo, bs;
+    float bs;
     unsigned first, span;
-    __device__ __forceinline__ SelTest(float klo_, float bs_, unsigned bin)
-        : klo(klo_), bs(bs_), first(kSelOne + bin),
+    __device__ __forceinline__ SelTest(float bs_, unsigned bin)
+        : bs(bs_), first(kSelOne + bin),
           span(bin == kSelBins - 1 ? 0xffffffffu - kSelOne - bin : 0u) {}
     __device__ __forceinline__ bool operator()(float k) const {
-        return __float_as_uint(fmaf(k - klo, bs, 8388608.f)) - first <= span;
+        return __float_as_uint(fmaf(k, bs, 8388608.f)) - first <= span;
     }
 };
 
@@ -198,50 +206,59 @@ __device__ __forceinline__ float sel_answer(SelScratch *sc, int count, unsigned 
 
 // Refinement of a crossing bin that held more than kSelList entries: `in` tells
 // its members among the line's elements e in [0, cnt) (samples xb[e], keys
-// keyfn(e, v)).  Each level finds the members' key range and histograms it.
+// keyfn(e, v)).  Each level histograms the bit patterns of the members' keys
+// (as integers in the floats' order; -0, of no weight, is below the range) from
+// the lowest to the highest, 256 bins: at most 31 bits to begin with and 8 fewer
+// after each level.  Not unrolled: that spilled in the callers' hot loops
+// (4096^2 x 720 angles, T0-T7: 66.3 ms, 64.8 rolled).
 template <class KeyFn, class WFn>
 __device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, WFn wfn,
                                          SelTest in, SelPick p, SelScratch *sc, int lane) {
-    float klo = 0.f, khi = 0.f;
-    for (int level = 0; level < 8; level++) {
-        // key range of the members (level > 0: of the last bin's, inside the
-        // last range)
-        float mn = __int_as_float(0x7f800000), mx = 0.f;
+    int lo = 0, hi = 0x7f800000; // the members' range
+    for (int level = 0; level < 5; level++) {
+        int mn = INT_MAX, mx = 0;
+#pragma unroll 1
         for (int e = lane; e < cnt; e += 32) {
-            const float v = xb[e], k = keyfn(e, v);
-            if (in(k) && (level == 0 || (k >= klo && k <= khi))) {
-                mn = fminf(mn, k);
-                mx = fmaxf(mx, k);
+            const float k = keyfn(e, xb[e]);
+            const int u = __float_as_int(k);
+            if (u >= lo && u <= hi && (level > 0 || in(k))) {
+                mn = min(mn, u);
+                mx = max(mx, u);
             }
         }
-        klo = __int_as_float(warp_min(__float_as_int(mn)));
-        khi = __int_as_float(warp_max(__float_as_int(mx)));
-        if (!(khi > klo))
-            return klo;
-        const float bs = (float)kSelBins / (khi - klo);
+        lo = __reduce_min_sync(TT_FULL_MASK, mn);
+        hi = __reduce_max_sync(TT_FULL_MASK, mx);
+        if (hi <= lo)
+            break;
+        const int shift = max(24 - __clz(hi - lo), 0);
         __syncwarp();
         sel_clear(sc, lane);
         __syncwarp();
+#pragma unroll 1
         for (int e = lane; e < cnt; e += 32) {
-            const float v = xb[e], k = keyfn(e, v);
-            if (k >= klo && k <= khi)
-                atomicAdd(sc->hist + sel_bin(k, klo, bs), wfn(v));
+            const float v = xb[e];
+            const int u = __float_as_int(keyfn(e, v));
+            if (u >= lo && u <= hi)
+                atomicAdd(sc->hist + ((u - lo) >> shift), wfn(v));
         }
         __syncwarp();
         p = sel_pick<false>(sc, p.below, p.total, lane);
-        in = SelTest(klo, bs, p.bin);
+        lo += (int)p.bin << shift;
+        hi = min(hi, lo + ((1 << shift) - 1));
         __syncwarp();
         int count = 0;
+#pragma unroll 1
         for (int e0 = 0; e0 < cnt; e0 += 32) {
             const int e = e0 + lane;
             const float v = e < cnt ? xb[e] : 0.f, k = keyfn(e, v);
-            sel_append(sc, count, e < cnt && k >= klo && k <= khi && in(k), k, v, lane);
+            const int u = __float_as_int(k);
+            sel_append(sc, count, e < cnt && u >= lo && u <= hi, k, v, lane);
         }
         __syncwarp();
         if (count <= kSelList)
             return sel_answer(sc, count, p.below, p.total, wfn, lane);
     }
-    return klo;
+    return __int_as_float(min(lo, hi));
 }
 
 // Clears a line's two histograms; before the team's next sync, which comes
@@ -288,7 +305,7 @@ __device__ __forceinline__ void select_t67(const float *x, int jlo, int jhi, int
     const SqrtWeight wfn{sel_scale(qtot), odd};
     const float k6max = __fmul_rn((float)max(jhi - 1 - m2, 0), xmax);
     want6 = want6 && k6max > 0.f; // otherwise every T6 key is 0
-    const float bs7 = (float)kSelBins / xmax, bs6 = want6 ? (float)kSelBins / k6max : 0.f;
+    const float bs7 = sel_per_key(xmax), bs6 = want6 ? sel_per_key(k6max) : 0.f;
     // element e of [0, cnt) is row b + e; this lane's are e0 .. e0 + mine - 1,
     // of which T7 takes those from i = f7 on and T6 those from f6
     const float *xb = x + (b - jlo);
@@ -311,9 +328,9 @@ __device__ __forceinline__ void select_t67(const float *x, int jlo, int jhi, int
             const unsigned wq = wfn(v); // 0 past the chunk
             l7max += v == xmax && i >= f7 ? wq : 0u;
             if (wq && i >= f7)
-                atomicAdd(s7->hist + sel_bin(v, 0.f, bs7), wq);
+                atomicAdd(s7->hist + sel_bin(v, bs7), wq);
             if (wq && i >= f6)
-                atomicAdd(s6->hist + sel_bin(__fmul_rn(rf + (float)u, v), 0.f, bs6), wq);
+                atomicAdd(s6->hist + sel_bin(__fmul_rn(rf + (float)u, v), bs6), wq);
         }
     }
     unsigned wtop = __reduce_add_sync(TT_FULL_MASK, l7max);
@@ -347,7 +364,7 @@ __device__ __forceinline__ void select_t67(const float *x, int jlo, int jhi, int
     }
     if (!want6 && !want7)
         return;
-    const SelTest in7(0.f, bs7, p7.bin), in6(0.f, bs6, p6.bin);
+    const SelTest in7(bs7, p7.bin), in6(bs6, p6.bin);
     int c6 = 0, c7 = 0;
     rf = r0;
     for (int i0 = 0; i0 < per; i0 += 4, rf += 4.f) {
@@ -408,7 +425,7 @@ inline __device__ float select_p2(const float *x, int n, float xmax, float xsum,
     const int per = ((n + 31) >> 5) | 1;
     const int j0 = lane * per, mine = min(max(n - j0, 0), per);
     const LinearWeight wfn{sel_scale(xsum)};
-    const float bs = (float)kSelBins / xmax;
+    const float bs = sel_per_key(xmax);
     sel_clear(sc, lane);
     __syncwarp();
     for (int i0 = 0; i0 < per; i0 += 4) { // warp-uniform trip count
@@ -420,13 +437,13 @@ inline __device__ float select_p2(const float *x, int n, float xmax, float xsum,
         for (int u = 0; u < 4; u++) {
             const unsigned wq = wfn(vb[u]);
             if (wq)
-                atomicAdd(sc->hist + sel_bin(vb[u], 0.f, bs), wq);
+                atomicAdd(sc->hist + sel_bin(vb[u], bs), wq);
         }
     }
     __syncwarp();
     const SelPick p = sel_pick<true>(sc, 0u, 0u, lane);
     __syncwarp();
-    const SelTest in(0.f, bs, p.bin);
+    const SelTest in(bs, p.bin);
     int c = 0;
     for (int i0 = 0; i0 < per; i0 += 4) {
         float vb[4];
