@@ -836,6 +836,13 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
         centers[s] = center + mx;
         max_m = std::max(max_m, m);
     }
+    // before any buffer moves: the graphs of other calls hold their addresses
+    if (max_m > tt::nos_max_rows())
+        return fail(TT_ERR_UNSUPPORTED,
+                    "nearest orthonormal sinogram of %d aligned rows exceeds %d", max_m,
+                    tt::nos_max_rows());
+    if (cols > 1024)
+        return fail(TT_ERR_UNSUPPORTED, "orthonormal circus of %d angles exceeds 1024", cols);
     for (NosDesc &d : desc) {
         d.ld = tt::nos_ld(d.m, max_m);
         d.a_off = (long long)a_elems;
@@ -851,12 +858,6 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
     TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, class_elems)));
     TT_CHECK(p->ensure(p->nos_desc, sizeof(NosDesc) * n_sino));
     TT_CHECK(p->ensure(p->nos, sizeof(float) * out_elems));
-    if (max_m > tt::nos_max_rows())
-        return fail(TT_ERR_UNSUPPORTED,
-                    "nearest orthonormal sinogram of %d aligned rows exceeds %d", max_m,
-                    tt::nos_max_rows());
-    if (cols > 1024)
-        return fail(TT_ERR_UNSUPPORTED, "orthonormal circus of %d angles exceeds 1024", cols);
     // scratch: 5 double-float + 3 int vectors of n, 3 float n x n matrices,
     // 2 float vectors, the sweep loop's state, then (256-byte aligned) the
     // sweeps' rotations and the Q application's
