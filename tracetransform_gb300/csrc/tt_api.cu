@@ -383,6 +383,14 @@ struct tt_plan {
         b.bytes = bytes;
         return TT_OK;
     }
+    // A buffer of `wanted` bytes, or of `needed` where the device has no room for that.
+    tt_status ensure(DevBuf &b, size_t wanted, size_t needed) {
+        const tt_status s = ensure(b, wanted);
+        if (s != TT_ERR_OOM || needed >= wanted)
+            return s;
+        cudaGetLastError(); // the refused allocation's
+        return ensure(b, needed);
+    }
     // Tables are created once and read by kernels on any stream, so the copy
     // completes before the table is handed out.
     template <typename T> tt_status upload(T **dst, const std::vector<T> &h) {
@@ -851,11 +859,12 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
         out_elems += (size_t)d.m * cols;
     }
     // the captured graphs hold these buffers' addresses, so they are sized for the
-    // longest columns of the row class: other images of a size then find
-    // them, and the graphs, as they are
+    // longest columns of the row class, where there is room: other images of a
+    // size then find them, and the graphs, as they are
     const int class_m = tt::nos_class_rows(max_m);
     const size_t class_elems = (size_t)tt::nos_ld(class_m, class_m) * ncol;
-    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, class_elems)));
+    TT_CHECK(p->ensure(p->nos_a, sizeof(float2) * std::max(a_elems, class_elems),
+                       sizeof(float2) * a_elems));
     TT_CHECK(p->ensure(p->nos_desc, sizeof(NosDesc) * n_sino));
     TT_CHECK(p->ensure(p->nos, sizeof(float) * out_elems));
     // scratch: 5 double-float + 3 int vectors of n, 3 float n x n matrices,
@@ -867,9 +876,11 @@ tt_status run_nos(tt_plan *p, const float *d_sino, int rows, int cols, int n_sin
                         sizeof(float) * n_sino + sizeof(unsigned) * 2;
     const size_t wy_at = (head + 255) & ~size_t(255);
     const size_t rotations = tt::nos_rotation_floats(cols, n_sino); // a multiple of 64
-    const size_t assemble = std::max(tt::nos_assemble_floats(cols, n_sino, max_m),
-                                     tt::nos_assemble_floats(cols, n_sino, class_m));
-    TT_CHECK(p->ensure(p->nos_work, wy_at + sizeof(float) * (rotations + assemble)));
+    const size_t assemble = tt::nos_assemble_floats(cols, n_sino, max_m);
+    const size_t class_assemble =
+        std::max(assemble, tt::nos_assemble_floats(cols, n_sino, class_m));
+    TT_CHECK(p->ensure(p->nos_work, wy_at + sizeof(float) * (rotations + class_assemble),
+                       wy_at + sizeof(float) * (rotations + assemble)));
     tt::NosWork w;
     {
         char *q = (char *)p->nos_work.p;
