@@ -53,19 +53,28 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) {
 template <bool kInv> __device__ __forceinline__ float2 crot(float2 a) {
     return kInv ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
-// a times exp(-+ 2 pi i / 16 * q) for the roots a radix-8 / 16 butterfly uses
+// a times exp(-+ 2 pi i / 16 * q) for the roots a radix-8 / 16 butterfly uses, the
+// roots as sums of two floats: unlike the table's twiddles, whose roundings
+// average out, these few enter every butterfly of every pass, and rounded to
+// floats they made P3 systematically small (by 1.8e-7 at 2049 rows, 0.5e-7 so).
+// Free: the passes wait for shared memory (5760 columns of 5793 rows 737 us
+// either way).
 template <bool kInv, int q> __device__ __forceinline__ float2 croot16(float2 a) {
-    constexpr float c1 = 0.923879532511286756f, s1 = 0.382683432365089772f,
-                    h = 0.707106781186547524f;
+    constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173,
+                     h = 0.70710678118654752440;
     if constexpr (q == 0)
         return a;
     else if constexpr (q == 4)
         return crot<kInv>(a);
     else {
-        constexpr float c = q == 1 ? c1 : q == 2 ? h : q == 3 ? s1 : q == 6 ? -h : -c1;
-        constexpr float s = q == 1 ? s1 : q == 2 ? h : q == 3 ? c1 : q == 6 ? h : -s1;
         static_assert(q == 1 || q == 2 || q == 3 || q == 6 || q == 9, "roots of the 4 x 4 split");
-        return kInv ? cmul(a, make_float2(c, s)) : cmul(a, make_float2(c, -s));
+        constexpr double re = q == 1 ? c1 : q == 2 ? h : q == 3 ? s1 : q == 6 ? -h : -c1;
+        constexpr double up = q == 1 ? s1 : q == 2 ? h : q == 3 ? c1 : q == 6 ? h : -s1;
+        constexpr double im = kInv ? up : -up;
+        constexpr float c = (float)re, cl = (float)(re - (double)c);
+        constexpr float s = (float)im, sl = (float)(im - (double)s);
+        return make_float2(fmaf(a.x, c, fmaf(-a.y, s, fmaf(a.x, cl, -a.y * sl))),
+                           fmaf(a.x, s, fmaf(a.y, c, fmaf(a.x, sl, a.y * cl))));
     }
 }
 
