@@ -2,7 +2,7 @@
 
 Runs maleadt/tracetransform's own c++/ sources, compiled unmodified against
 the stand-in headers in oracle/shim/ (``make -C oracle ref``; needs a checkout
-of the reference, by default /root/reference), on seeded synthetic images and
+of the reference, whose folder REF names), on seeded synthetic images and
 stores inputs and outputs as compressed .npz files:
 
     python tests/golden/make_golden.py        # transform / rotate fixtures

@@ -200,10 +200,10 @@ __global__ void circus_backward_kernel(const T *__restrict__ sino, int rows, int
 // and n / 2) the sums are real, so they are the real and the negated
 // imaginary part of DFT(conj(G1 + i G2)).  Columns (and their W) enter with
 // norms of about one; where a squared norm is not a normal float (that of W goes
-// with the sixth power of the column) each column takes transforms of its own.  Dynamic shared memory: the transform's buffer, then
-// W of both columns (n/2 + 1 pairs each).  64 x 3 x 360 columns of 363 rows
-// (with the rest of their training step): 14.9 ms, against 18.7 ms with
-// radix-2 passes on single columns (512 threads, 40 barriers; 4.2 ms alone).
+// with the sixth power of the column) each column takes transforms of its own.
+// Dynamic shared memory: the transform's buffer, then W of both columns (n/2 + 1
+// pairs each).  64 x 3 x 360 columns of 363 rows: 0.44 ms, from 4.20 ms with
+// radix-2 passes on single columns (512 threads, 40 barriers).
 template <int LOGM>
 __global__ void __launch_bounds__(fft_threads(LOGM))
 circus_backward_fft_kernel(const float *__restrict__ sino, int n, int cols,

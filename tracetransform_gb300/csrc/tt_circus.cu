@@ -702,7 +702,7 @@ struct P3FftArgs {
 // CTA per pair (tt_fft.cuh).  Both columns are brought to norms of about one
 // by powers of two first; a column whose squared norm is not a normal float
 // keeps out of its neighbour's transform and takes one of its own.  P1-P3 of
-// 5760 columns of 5793 rows: 0.82 ms (6.12 ms with one column per CTA in 28
+// 5760 columns of 5793 rows: 0.74 ms (6.12 ms with one column per CTA in 28
 // barrier-bound radix-2 passes).
 template <int LOGM>
 __global__ void __launch_bounds__(fft_threads(LOGM)) p3_fft_pair_kernel(const P3FftArgs a) {

@@ -57,8 +57,9 @@ template <bool kInv> __device__ __forceinline__ float2 crot(float2 a) {
 // roots as sums of two floats: unlike the table's twiddles, whose roundings
 // average out, these few enter every butterfly of every pass, and rounded to
 // floats they made P3 systematically small (by 1.8e-7 at 2049 rows, 0.5e-7 so).
-// Free: the passes wait for shared memory (5760 columns of 5793 rows 737 us
-// either way).
+// Where the passes wait for shared memory this costs nothing (P1-P3 of 5760 columns
+// of 5793 rows 737 us either way); the adjoint of 69120 columns of 363 rows takes
+// 441 us, from 430.
 template <bool kInv, int q> __device__ __forceinline__ float2 croot16(float2 a) {
     constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173,
                      h = 0.70710678118654752440;

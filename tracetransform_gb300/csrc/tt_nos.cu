@@ -334,11 +334,12 @@ template <int GB> __device__ __forceinline__ float2 qr_warp_sums(float2 (&v)[GB]
 // two lanes.  Sums, updates and scalars are all double-float; their order
 // hangs on T alone (polar factors of nearly dependent columns change visibly
 // with their last bits).
-// The whole orthonormal circus, before (an address and a row test per access, a
-// reduction and a barrier per column) and after this alone: 8 x 1449 x 360, 9.28 and
-// 8.4; 4 x 450 x 360, 6.16 and 5.6; 8 x 5795 x 720, 90.6 and 87.  Two rows at a time in packed
-// operations took 40 % fewer instructions and as long: a step then waits for its
-// chain.
+// The whole orthonormal circus with an address and a row test per access, a
+// reduction and a barrier per column, then by this alone, then with the other
+// kernels of this file as they are now: 8 x 1449 x 360, 9.28, 8.4 and 7.90 ms;
+// 4 x 450 x 360, 6.2, 5.6 and 4.89; 8 x 5793 x 720, 90.6, 87 and 85.6.  Two rows at a
+// time in packed operations took 40 % fewer instructions and as long: a step then
+// waits for its chain.
 //
 // K: rows per thread.  CTAs per SM: by registers (two floats per row of x, and
 // more to have the column's loads in flight: bounds of 5 and 3 CTAs for K = 16 took
@@ -937,10 +938,11 @@ rt_block_round_kernel(float *__restrict__ X, float *__restrict__ J, int n, int n
 // 4 columns of a block pair, 24 steps of two 16-byte loads and 16
 // multiply-adds; the CTA's warps share the J's, staged 16 pairs (3 tiles
 // per lane) ahead.  Runs beside the next sweep's rounds, which are chains that leave
-// most of the machine idle.  Orthonormal circus with V rotated inside the rounds, and
-// so: 4 x 450 x 360, 5.56 and 4.97 ms; 8 x 1449 x 360, 8.04 and 7.79; 8 x 5795 x 720,
-// 77.3 and 76.7.  Keeping the rounds' CTAs off its SMs (one CTA with all the shared
-// memory on each SM they leave) measured slower, 7.85 at 8 x 1449 x 360.
+// most of the machine idle.  Against V rotated inside the rounds the orthonormal
+// circus gained 0.6 ms of 5.6 at 4 x 450 x 360, 0.25 of 8.0 at 8 x 1449 x 360 and 0.6
+// of 77 at 8 x 5795 x 720 (with a QR that summed in another order).  Keeping the
+// rounds' CTAs off its SMs (one CTA with all the shared memory on each SM they
+// leave) took 0.06 ms longer at 8 x 1449 x 360.
 // grid (ceil(n / (4 warps)), n_sino).
 constexpr int kVMaxWarps = 8, kVPairs = 16, kVPairLd = kBJFloats + 24; // pairs 24 banks apart
 constexpr int kVTiles = kVPairs * (kBCols / 4) / 32;
@@ -1707,8 +1709,8 @@ static cudaError_t qr_steps(float2 *A, const NosDesc *desc, int n, int n_sino, c
     for (int k = 0; k < n; k++) {
         // CTAs of one column while that makes at most 6 per SM, of whole groups above:
         // the work a CTA does whatever its columns then counts for more than
-        // the chain over them (1 x 1449 x 360, 5.36 against 5.67 ms in all with
-        // groups; 4 x 450 x 360, 5.87 against 5.70)
+        // the chain over them (1 x 1449 x 360, 0.31 ms less in all than with groups;
+        // 4 x 450 x 360, 0.17 more)
         const long long left = n - k;
         const long long g =
             left * n_sino <= 6LL * sms ? left : (left + kQrGroup - 1) / kQrGroup;
@@ -1805,8 +1807,8 @@ size_t nos_rotation_floats(int n, int n_sino) {
 }
 
 // Eight warps per CTA where the sweeps' rounds fill the machine (fewer copies of the
-// J's: 76.5 against 78.3 ms at 8 x 5795 x 720), else four (7.78 against 7.90 at
-// 8 x 1449 x 360).
+// J's: 1.8 ms less of the orthonormal circus at 8 x 5795 x 720 than with four), else
+// four (0.12 ms less at 8 x 1449 x 360).
 static cudaError_t rotate_v(int n, int n_sino, const NosWork &w, cudaStream_t st) {
     const int nbp = nos_blocks(n);
     int dev = 0, sms = 0;

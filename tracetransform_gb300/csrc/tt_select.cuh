@@ -22,9 +22,10 @@
 // element as it needs -- bins by one multiply-add into the mantissa of 2^23,
 // weights (a square root each) only in the histogram pass and for the few
 // collected entries -- and the fixed work per line.  The collected list takes
-// the histogram's place in shared memory.  1024^2 x 360 angles, T0-T7: 2.55 ms
-// (3.21 with the bins recomputed by conversions and the weights in both
-// passes, 64-bit scans and a 64-entry bitonic sort).
+// the histogram's place in shared memory.  The sinogram kernel at 1024^2 x 360
+// angles, T0-T7, by this alone: 2.55 ms, from 3.21 with the bins recomputed by
+// conversions and the weights in both passes, 64-bit scans and a 64-entry bitonic
+// sort (2.07 with the roots and the sampling since).
 #pragma once
 
 #include <climits>
@@ -210,7 +211,7 @@ __device__ __forceinline__ float sel_answer(SelScratch *sc, int count, unsigned 
 // (as integers in the floats' order; -0, of no weight, is below the range) from
 // the lowest to the highest, 256 bins: at most 31 bits to begin with and 8 fewer
 // after each level.  Not unrolled: that spilled in the callers' hot loops
-// (4096^2 x 720 angles, T0-T7: 66.3 ms, 64.8 rolled).
+// (4096^2 x 720 angles, T0-T7: 66.3 ms, 65.3 rolled).
 template <class KeyFn, class WFn>
 __device__ __noinline__ float sel_refine(const float *xb, int cnt, KeyFn keyfn, WFn wfn,
                                          SelTest in, SelPick p, SelScratch *sc, int lane) {
