@@ -365,13 +365,16 @@ __device__ __forceinline__ int stack_of(const CircusStack *st, int n_st, int v, 
 // out) makes the tile's partial sums NaN instead of hanging the GPU.
 //
 // Bound: shared-memory bandwidth -- the MMAs read 96 KB a stage and the fills
-// write 64, 1280 cycles of about 2200.  2880 columns of 1449: 105 us (116 with
-// the thread-per-column loads).
+// write 64, 1280 cycles of about 2200.  P3 of 2880 columns of 1449 rows, the whole call: 108 us
+// (124 with the thread-per-column loads, 114 when a producer also started the
+// twiddle copies).  Of 45 columns, where no stage has anything else to wait for than
+// its copy: 61 us (61, 65).
 constexpr int kTcCols = 128, kTcKT = 32, kTcThreads = 256, kTcN = 2 * kFreqTile;
 constexpr int kTcAcc = 4; // accumulators of kTcN columns: hi.hi x 3, cross terms
 constexpr int kTcAFloats = kTcCols * kTcKT, kTcBFloats = kTcN * kTcKT;
 constexpr size_t kTcBufFloats = 2 * (size_t)kTcAFloats + 2 * (size_t)kTcBFloats;
 constexpr int kTcRing = 3; // stage buffers
+constexpr int tc_threads(bool pre) { return kTcThreads + (pre ? 64 : 32); }
 constexpr size_t kTcSmem = kTcRing * kTcBufFloats * sizeof(float); // 192 KB
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
@@ -463,15 +466,17 @@ __global__ void p3_tc_tables_kernel(int n, const float2 *__restrict__ tw, float 
 
 // grid: one CTA per (64-frequency tile, 128 columns) over the stacks.
 // Warp-specialised: warps 0-7 produce the stages into a ring of kTcRing
-// buffers (each thread its 16 sinogram samples, hi / lo split and stored;
-// with kPre one thread also starts the bulk copy of the twiddle blocks) and
-// arrive on the slot's `full` barrier (256 arrivals plus the copy's bytes);
-// warp 8 waits on `full`, issues the slot's 12 MMAs and commits them to the
-// slot's `empty` barrier, which the producers wait on before refilling it.
+// buffers (each thread its 16 sinogram samples, hi / lo split and stored) and
+// arrive on the slot's `full` barrier (256 arrivals); with kPre warp 9 starts the
+// bulk copy of the slot's twiddle blocks (one more arrival and the copy's bytes) as
+// soon as the slot is empty, which a producer would do only once its own
+// samples are there; warp 8 waits on `full`, issues the slot's 12 MMAs and
+// commits them to the slot's `empty` barrier, which the producers wait on
+// before refilling it.
 // No CTA barrier inside the stage loop: producers run up to kTcRing stages
 // ahead of the MMAs.  Warps 0-3 then read the accumulators.
 template <bool kPre>
-__global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const CircusStackArgs a) {
+__global__ void __launch_bounds__(tc_threads(kPre), 1) p3_dft_tc_kernel(const CircusStackArgs a) {
     extern __shared__ __align__(1024) float tsm[];
     __shared__ __align__(8) unsigned long long s_full[kTcRing], s_empty[kTcRing], s_done;
     __shared__ unsigned s_tmem;
@@ -496,7 +501,7 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
     if (tid == 0) {
         for (int i = 0; i < kTcRing; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&s_full[i])),
-                         "r"((unsigned)kTcThreads)
+                         "r"((unsigned)(kTcThreads + (kPre ? 1 : 0)))
                          : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&s_empty[i])),
                          "r"(1u)
@@ -543,6 +548,24 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
                              smem_addr(&s_done))
                          : "memory");
         }
+    } else if (warp > kMmaWarp) { // the twiddle blocks (hi, lo: contiguous here and there)
+        if (lane == 0)
+            for (int s = 0; s < stages; s++) {
+                const int b = s % kTcRing;
+                if (s >= kTcRing)
+                    ok &= mbar_wait(smem_addr(&s_empty[b]), (unsigned)(s / kTcRing - 1) & 1u);
+                const unsigned bytes = (unsigned)(2 * kTcBFloats * sizeof(float));
+                unsigned long long state;
+                asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 %0, [%1], %2;"
+                             : "=l"(state)
+                             : "r"(smem_addr(&s_full[b])), "r"(bytes)
+                             : "memory");
+                const float *src = S.wtc + ((size_t)mt * stages + s) * 2 * kTcBFloats;
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 smem_addr(tsm + b * kTcBufFloats + 2 * kTcAFloats)),
+                             "l"(src), "r"(bytes), "r"(smem_addr(&s_full[b]))
+                             : "memory");
+            }
     } else {
         // producers.  Sinogram operand: warp w brings columns 16 w .. + 15, a
         // lane one sample of the stage's 32, so that a load reads 128
@@ -604,18 +627,6 @@ __global__ void __launch_bounds__(kTcThreads + 32, 1) p3_dft_tc_kernel(const Cir
                 fetch((s + 1) * kTcKT);
             if (s >= kTcRing)
                 ok &= mbar_wait(smem_addr(&s_empty[b]), (unsigned)(s / kTcRing - 1) & 1u);
-            if (kPre && tid == 0) { // the stage's twiddle blocks (hi, lo: contiguous here and there)
-                const unsigned bytes = (unsigned)(2 * kTcBFloats * sizeof(float));
-                asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(
-                                 smem_addr(&s_full[b])),
-                             "r"(bytes)
-                             : "memory");
-                const float *src = S.wtc + ((size_t)mt * stages + s) * 2 * kTcBFloats;
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                 smem_addr(Bhi)),
-                             "l"(src), "r"(bytes), "r"(smem_addr(&s_full[b]))
-                             : "memory");
-            }
 #pragma unroll
             for (int i = 0; i < 16; i++) {
                 const int at = (16 * warp + i) * 32 + (lane ^ (4 * (i & 7)));
@@ -992,9 +1003,9 @@ cudaError_t launch_circus_stacks(const CircusStackArgs &a, size_t smem, cudaStre
         if (opt_in_smem(k) < kTcSmem)
             return cudaErrorInvalidValue;
         if (a.tc_tables)
-            p3_dft_tc_kernel<true><<<a.total_tiles, kTcThreads + 32, kTcSmem, st>>>(a);
+            p3_dft_tc_kernel<true><<<a.total_tiles, tc_threads(true), kTcSmem, st>>>(a);
         else
-            p3_dft_tc_kernel<false><<<a.total_tiles, kTcThreads + 32, kTcSmem, st>>>(a);
+            p3_dft_tc_kernel<false><<<a.total_tiles, tc_threads(false), kTcSmem, st>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return e;
     }
