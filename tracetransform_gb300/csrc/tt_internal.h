@@ -117,8 +117,8 @@ cudaError_t launch_p3_tc_tables(int n, const float2 *tw, float *out, cudaStream_
 // The line dates from transforms of single columns in radix-2 passes, and the
 // batch and the allocation-free entry point have the direct DFT alone, whose
 // results the single call's are compared with.  Column pairs of radix-16 passes
-// are the faster from 256 rows up (P3 of 2880 columns: 256 rows 26 and 23 us, 1024
-// rows 88 and 40, 1449 rows 116 and 60, 2048 rows 217 and 64).
+// are the faster from 256 rows up (P3 of 2880 columns: 256 rows 26 and 23 us, 1449
+// rows 108 and 60, 2048 rows 199 and 64).
 constexpr int kP3DftMaxRows = 2048;
 // P3 of longer columns by the chirp-z transform of column pairs, into entries
 // p with kind[p] == 3 of out (n_sino x n_p x cols); only where fft_pair_fits(M).
